@@ -35,8 +35,8 @@ constexpr int NIN = CT2G_MLP_NIN, NH = CT2G_MLP_NHID, NP = CT2G_MLP_NPARAM;
 constexpr int OW1 = 0, OB1 = OW1 + NH * NIN, OW2 = OB1 + NH, OB2 = OW2 + NH * NH,
               OW3 = OB2 + NH, OB3 = OW3 + NH;
 static_assert(OB3 + 1 == NP, "parameter layout");
-// per-sample values kept for the weight gradients: h1 | dz1 | h2 | dz2 | dy
-constexpr int kStash = 4 * NH + 4;
+// a block's partial gradient sums: the parameters, then the squared error
+constexpr int NPL = NP + 1;
 
 }  // namespace
 
@@ -87,10 +87,10 @@ struct ct2g_learn {
   // training set
   float *tX = nullptr, *tT = nullptr;
   size_t tn = 0, tcap = 0;
-  float *stash = nullptr;      // [batch][kStash]
-  float *sloss = nullptr;      // [batch]
+  float *gpart = nullptr;      // [gradient blocks][NPL] partial sums
   uint32_t *tidx = nullptr;    // [tcap] sample order
-  size_t stash_cap = 0;
+  float *gX = nullptr, *gT = nullptr;  // ct2g_mlp_gradients' samples on the device
+  size_t g_cap = 0;
 };
 
 namespace {
@@ -330,97 +330,262 @@ __global__ void __launch_bounds__(256) mlp_infer_kernel(
   }
 }
 
-// forward + backward of samples idx[start .. start+count): per sample the
-// hidden activations and the errors go to the stash (h1 | dz1 | h2 | dz2 |
-// dy), the squared error to sloss.  dL/dy = 2 (y - t) / count (mean squared
-// error); the ReLU derivatives are kept as bit masks.
-__global__ void __launch_bounds__(128) mlp_fwdbwd_kernel(
-    const __nv_bfloat16 *__restrict__ wbf, const float *__restrict__ fmean,
-    const float *__restrict__ fstd, const float *__restrict__ X, const float *__restrict__ T,
-    const uint32_t *__restrict__ idx, size_t start, int count, float *__restrict__ stash,
-    float *__restrict__ sloss) {
-  extern __shared__ float ws[];
-  load_weights(ws, wbf);
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= count) return;
-  const uint32_t q = idx[start + s];
-  float x[NIN];
+// Loss and gradient of samples idx[start .. start+count) (idx null: start ..
+// start+count): forward, backward and weight gradients of a tile of 64
+// samples by one block, the activations and errors never leaving shared
+// memory.  The products are 64 x 64 x {24, 64} matrix products in FP32 (BF16
+// weights, FP32 activations and sums, so the CUDA cores, not the tensor cores),
+// 256 threads as 16 x 16 with a 4 x 4 register tile each: 16 FMAs per two
+// 16-byte shared loads, 16 independent sums against the FMA latency.  Arrays are
+// [feature][sample] with 68 floats per row: rows tx, tx + 16, ... read four
+// samples at a time hit every bank once per quarter warp.  A block keeps its
+// weight gradients in registers over its tiles (stride gridDim.x) and writes
+// one partial sum per parameter; mlp_reduce_kernel adds the blocks' in a fixed order, so
+// the result is the same on every run.  dL/dy = 2 (y - t) / count (mean
+// squared error).
+//
+// What bounds it: 6 x 5696 FLOP per sample, 0.7 GFLOP at 20,011 samples (9 us
+// of the FP32 peak); the kernels it replaces gave a whole weight's sum over the
+// samples to one thread (5825 threads on the chip, each a serial chain of
+// loads: 7.47 ms).  ct2g_mlp_gradients at 20,011 samples: 7.64 -> 0.235 ms a
+// call, most of it the host copies of the samples.
+constexpr int TS = 64;          // samples per tile
+constexpr int TP = TS + 4;      // floats per row of a tile array
+struct GradSmem {
+  float w1[NIN][NH];            // [i][slot(j)]: slot(j) = 4 (j % 16) + j / 16, so that a
+                                // thread's rows tx + 16 q are one 16-byte load
+  float w2[NH][NH];             // [k][slot(j)] = W2[j][k]
+  float w2t[NH][NH];            // [j][slot(k)] = W2[j][k]
+  float b1[NH], b2[NH], w3[NH];
+  float x[NIN][TP];             // normalised inputs
+  float h1[NH][TP];             // hidden 1, then its errors dz1
+  float h2[NH][TP];             // hidden 2, then its errors dz2
+  float dy[TS];
+};
+
+// acc[q][u] += sum_s a[tx + 16 q][s] b[ty + 16 u][s] over a tile's samples
+template <int U>
+__device__ __forceinline__ void outer_sum(const float (*a)[TP], const float (*b)[TP], int tx,
+                                          int ty, int nb, float (&acc)[4][U]) {
+#pragma unroll 2
+  for (int s = 0; s < TS; s += 4) {
+    float4 av[4], bv[U];
 #pragma unroll
-  for (int i = 0; i < NIN; i++) x[i] = (X[(size_t)q * NIN + i] - fmean[i]) / fstd[i];
-  float *st = stash + (size_t)s * kStash;
-  float h1[NH];
-  unsigned long long m1 = 0ull, m2 = 0ull;
+    for (int q = 0; q < 4; q++) av[q] = *reinterpret_cast<const float4 *>(&a[tx + 16 * q][s]);
 #pragma unroll
-  for (int j = 0; j < NH; j++) {
-    float a = ws[OB1 + j];
+    for (int u = 0; u < U; u++)
+      bv[u] = ty + 16 * u < nb ? *reinterpret_cast<const float4 *>(&b[ty + 16 * u][s])
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < NIN; i++) a = fmaf(ws[OW1 + j * NIN + i], x[i], a);
-    h1[j] = fmaxf(a, 0.f);
-    if (a > 0.f) m1 |= 1ull << j;
-    st[j] = h1[j];
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        acc[q][u] = fmaf(av[q].x, bv[u].x, acc[q][u]);
+        acc[q][u] = fmaf(av[q].y, bv[u].y, acc[q][u]);
+        acc[q][u] = fmaf(av[q].z, bv[u].z, acc[q][u]);
+        acc[q][u] = fmaf(av[q].w, bv[u].w, acc[q][u]);
+      }
   }
-  float y = ws[OB3];
-#pragma unroll 1
-  for (int j = 0; j < NH; j++) {
-    float a = ws[OB2 + j];
-#pragma unroll
-    for (int k = 0; k < NH; k++) a = fmaf(ws[OW2 + j * NH + k], h1[k], a);
-    if (a > 0.f) m2 |= 1ull << j;
-    st[2 * NH + j] = fmaxf(a, 0.f);
-    y = fmaf(ws[OW3 + j], fmaxf(a, 0.f), y);
-  }
-  const float e = y - T[q];
-  sloss[s] = e * e;
-  const float dy = 2.f * e / (float)count;
-  st[4 * NH] = dy;
-  float dz1[NH];
-#pragma unroll
-  for (int k = 0; k < NH; k++) dz1[k] = 0.f;
-#pragma unroll 1
-  for (int j = 0; j < NH; j++) {
-    const float dz2 = ((m2 >> j) & 1ull) ? dy * ws[OW3 + j] : 0.f;
-    st[3 * NH + j] = dz2;
-#pragma unroll
-    for (int k = 0; k < NH; k++) dz1[k] = fmaf(ws[OW2 + j * NH + k], dz2, dz1[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < NH; k++) st[NH + k] = ((m1 >> k) & 1ull) ? dz1[k] : 0.f;
 }
 
-// weight gradients, one thread per parameter, summed over the batch in a
-// fixed order (deterministic)
-__global__ void mlp_wgrad_kernel(const float *__restrict__ fmean, const float *__restrict__ fstd,
-                                 const float *__restrict__ X, const uint32_t *__restrict__ idx,
-                                 size_t start, int count, const float *__restrict__ stash,
-                                 float *__restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= NP) return;
-  float g = 0.f;
-  if (p < OB1) {
-    const int j = p / NIN, i = p % NIN;
-    const float m = fmean[i], sd = fstd[i];
-    for (int s = 0; s < count; s++) {
-      const float x = (X[(size_t)idx[start + s] * NIN + i] - m) / sd;
-      g = fmaf(stash[(size_t)s * kStash + NH + j], x, g);
+// v[q][u] = init[tx + 16 q] + sum_k w[k][slot(tx + 16 q)] a[k][4 ty + u], k
+// in order (init null: 0)
+template <int K>
+__device__ __forceinline__ void layer(const float (*w)[NH], const float (*a)[TP],
+                                      const float *init, int tx, int ty, float (&v)[4][4]) {
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[q][u] = init ? init[tx + 16 * q] : 0.f;
+#pragma unroll 4
+  for (int k = 0; k < K; k++) {
+    const float4 wv = *reinterpret_cast<const float4 *>(&w[k][4 * tx]);
+    const float4 av = *reinterpret_cast<const float4 *>(&a[k][4 * ty]);
+    const float wq[4] = {wv.x, wv.y, wv.z, wv.w}, au[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[q][u] = fmaf(wq[q], au[u], v[q][u]);
+  }
+}
+
+__device__ __forceinline__ int wslot(int j) { return 4 * (j & 15) + (j >> 4); }
+
+__global__ void __launch_bounds__(256, 2) mlp_grad_kernel(
+    const __nv_bfloat16 *__restrict__ wbf, const float *__restrict__ fmean,
+    const float *__restrict__ fstd, const float *__restrict__ X, const float *__restrict__ T,
+    const uint32_t *__restrict__ idx, size_t start, int count, float *__restrict__ part) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  GradSmem &sm = *reinterpret_cast<GradSmem *>(smraw);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int i = tid; i < NH * NIN; i += 256)
+    sm.w1[i % NIN][wslot(i / NIN)] = __bfloat162float(wbf[OW1 + i]);
+  for (int i = tid; i < NH * NH; i += 256) {
+    const int j = i / NH, k = i % NH;
+    const float w = __bfloat162float(wbf[OW2 + i]);
+    sm.w2[k][wslot(j)] = w;
+    sm.w2t[j][wslot(k)] = w;
+  }
+  if (tid < NH) {
+    sm.b1[tid] = __bfloat162float(wbf[OB1 + tid]);
+    sm.b2[tid] = __bfloat162float(wbf[OB2 + tid]);
+    sm.w3[tid] = __bfloat162float(wbf[OW3 + tid]);
+  }
+  const float b3 = __bfloat162float(wbf[OB3]);
+  float g1[4][2] = {}, g2[4][4] = {};  // W1[tx + 16 q][ty + 16 u], W2[tx + 16 q][ty + 16 u]
+  // thread j < 64: b1[j]; 64 + j: b2[j]; 128 + j: W3[j]; 192: b3
+  float gv = 0.f, se = 0.f;            // se: squared errors of sample slot tid
+  const int ntile = (count + TS - 1) / TS;
+  for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
+    const int n = min(TS, count - t * TS);
+    __syncthreads();
+    for (int e = tid; e < TS * NIN; e += 256) {
+      const int s = e / NIN, i = e - s * NIN;
+      float v = 0.f;
+      if (s < n) {
+        const size_t o = start + (size_t)t * TS + s;
+        const size_t q = idx ? idx[o] : o;
+        v = (X[q * NIN + i] - fmean[i]) / fstd[i];
+      }
+      sm.x[i][s] = v;
     }
-  } else if (p < OW2) {
-    const int j = p - OB1;
-    for (int s = 0; s < count; s++) g += stash[(size_t)s * kStash + NH + j];
-  } else if (p < OB2) {
-    const int j = (p - OW2) / NH, k = (p - OW2) % NH;
-    for (int s = 0; s < count; s++)
-      g = fmaf(stash[(size_t)s * kStash + 3 * NH + j], stash[(size_t)s * kStash + k], g);
-  } else if (p < OW3) {
-    const int j = p - OB2;
-    for (int s = 0; s < count; s++) g += stash[(size_t)s * kStash + 3 * NH + j];
-  } else if (p < OB3) {
-    const int k = p - OW3;
-    for (int s = 0; s < count; s++)
-      g = fmaf(stash[(size_t)s * kStash + 4 * NH], stash[(size_t)s * kStash + 2 * NH + k], g);
-  } else {
-    for (int s = 0; s < count; s++) g += stash[(size_t)s * kStash + 4 * NH];
+    __syncthreads();
+    float v[4][4];
+    layer<NIN>(sm.w1, sm.x, sm.b1, tx, ty, v);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      *reinterpret_cast<float4 *>(&sm.h1[tx + 16 * q][4 * ty]) =
+          make_float4(fmaxf(v[q][0], 0.f), fmaxf(v[q][1], 0.f), fmaxf(v[q][2], 0.f),
+                      fmaxf(v[q][3], 0.f));
+    __syncthreads();
+    layer<NH>(sm.w2, sm.h1, sm.b2, tx, ty, v);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      *reinterpret_cast<float4 *>(&sm.h2[tx + 16 * q][4 * ty]) =
+          make_float4(fmaxf(v[q][0], 0.f), fmaxf(v[q][1], 0.f), fmaxf(v[q][2], 0.f),
+                      fmaxf(v[q][3], 0.f));
+    __syncthreads();
+    if (tid < TS) {
+      float y = b3;
+#pragma unroll 8
+      for (int j = 0; j < NH; j++) y = fmaf(sm.w3[j], sm.h2[j][tid], y);
+      float dy = 0.f;
+      if (tid < n) {
+        const size_t o = start + (size_t)t * TS + tid;
+        const float e = y - T[idx ? idx[o] : o];
+        se += e * e;
+        dy = 2.f * e / (float)count;
+      }
+      sm.dy[tid] = dy;
+    }
+    __syncthreads();
+    if (tid >= 128 && tid < 192) {
+      const int k = tid - 128;
+#pragma unroll 4
+      for (int s = 0; s < TS; s += 4) {
+        const float4 d = *reinterpret_cast<const float4 *>(&sm.dy[s]);
+        const float4 h = *reinterpret_cast<const float4 *>(&sm.h2[k][s]);
+        gv = fmaf(d.x, h.x, gv);
+        gv = fmaf(d.y, h.y, gv);
+        gv = fmaf(d.z, h.z, gv);
+        gv = fmaf(d.w, h.w, gv);
+      }
+    } else if (tid == 192) {
+      for (int s = 0; s < TS; s++) gv += sm.dy[s];
+    }
+    __syncthreads();
+    // errors of hidden 2 over its activations (own elements only); the rectifier
+    // passes where the activation is positive
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float w = sm.w3[tx + 16 * q];
+      float4 *p = reinterpret_cast<float4 *>(&sm.h2[tx + 16 * q][4 * ty]);
+      const float4 h = *p, d = *reinterpret_cast<const float4 *>(&sm.dy[4 * ty]);
+      *p = make_float4(h.x > 0.f ? d.x * w : 0.f, h.y > 0.f ? d.y * w : 0.f,
+                       h.z > 0.f ? d.z * w : 0.f, h.w > 0.f ? d.w * w : 0.f);
+    }
+    __syncthreads();
+    outer_sum<4>(sm.h2, sm.h1, tx, ty, NH, g2);
+    if (tid >= 64 && tid < 128)
+      for (int s = 0; s < TS; s++) gv += sm.h2[tid - 64][s];
+    layer<NH>(sm.w2t, sm.h2, nullptr, tx, ty, v);
+    float4 hm[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      hm[q] = *reinterpret_cast<const float4 *>(&sm.h1[tx + 16 * q][4 * ty]);
+    __syncthreads();  // every reader of hidden 1 done: its errors take its place
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      *reinterpret_cast<float4 *>(&sm.h1[tx + 16 * q][4 * ty]) =
+          make_float4(hm[q].x > 0.f ? v[q][0] : 0.f, hm[q].y > 0.f ? v[q][1] : 0.f,
+                      hm[q].z > 0.f ? v[q][2] : 0.f, hm[q].w > 0.f ? v[q][3] : 0.f);
+    __syncthreads();
+    outer_sum<2>(sm.h1, sm.x, tx, ty, NIN, g1);
+    if (tid < 64)
+      for (int s = 0; s < TS; s++) gv += sm.h1[tid][s];
+  }
+  float *p = part + (size_t)blockIdx.x * NPL;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (ty + 16 * u < NIN) p[OW1 + (tx + 16 * q) * NIN + ty + 16 * u] = g1[q][u];
+#pragma unroll
+    for (int u = 0; u < 4; u++) p[OW2 + (tx + 16 * q) * NH + ty + 16 * u] = g2[q][u];
+  }
+  if (tid < 64) p[OB1 + tid] = gv;
+  else if (tid < 128) p[OB2 + tid - 64] = gv;
+  else if (tid < 192) p[OW3 + tid - 128] = gv;
+  else if (tid == 192) p[OB3] = gv;
+  // the block's squared error: the 64 sample slots' sums
+  __syncthreads();
+  if (tid < TS) sm.dy[tid] = se;
+  __syncthreads();
+  if (tid == 0) {
+    float a = 0.f;
+    for (int s = 0; s < TS; s++) a += sm.dy[s];
+    p[NP] = a;
+  }
+}
+
+// The blocks' partial sums added in a fixed order: 32 parameters per block, 8
+// slices of the partials each (coalesced rows), then the slices.  grad[NP] =
+// the mean squared error.  lr > 0: the Adam step of the parameter follows in
+// place (adam_step), so an optimisation batch is two launches.
+struct AdamArgs {
+  float *p, *m, *v;
+  __nv_bfloat16 *wbf;
+  float lr, c1, c2;
+};
+__device__ __forceinline__ void adam_step(const AdamArgs &a, int i, float g) {
+  const float b1 = 0.9f, b2 = 0.999f;
+  a.m[i] = b1 * a.m[i] + (1.f - b1) * g;
+  a.v[i] = b2 * a.v[i] + (1.f - b2) * g * g;
+  a.p[i] -= a.lr * (a.m[i] / a.c1) / (sqrtf(a.v[i] / a.c2) + 1e-8f);
+  a.wbf[i] = __float2bfloat16_rn(a.p[i]);
+}
+__global__ void __launch_bounds__(256) mlp_reduce_kernel(const float *__restrict__ part, int nblk,
+                                                         int count, float *__restrict__ grad,
+                                                         AdamArgs adam) {
+  __shared__ float s[8][32];
+  const int l = threadIdx.x & 31, sl = threadIdx.x >> 5, p = blockIdx.x * 32 + l;
+  float a = 0.f;
+  if (p < NPL) {
+#pragma unroll 4
+    for (int b = sl; b < nblk; b += 8) a += part[(size_t)b * NPL + p];
+  }
+  s[sl][l] = a;
+  __syncthreads();
+  if (sl || p >= NPL) return;
+  float g = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; k++) g += s[k][l];
+  if (p == NP) {
+    grad[NP] = g / (float)count;
+    return;
   }
   grad[p] = g;
+  if (adam.lr > 0.f) adam_step(adam, p, g);
 }
 
 }  // namespace
@@ -786,34 +951,9 @@ __global__ void norm_stats_kernel(const float *__restrict__ X, size_t n, float *
   }
 }
 
-__global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                            float *__restrict__ v, __nv_bfloat16 *__restrict__ wbf, float lr,
-                            float c1, float c2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= NP) return;
-  const float b1 = 0.9f, b2 = 0.999f;
-  m[i] = b1 * m[i] + (1.f - b1) * g[i];
-  v[i] = b2 * v[i] + (1.f - b2) * g[i] * g[i];
-  p[i] -= lr * (m[i] / c1) / (sqrtf(v[i] / c2) + 1e-8f);
-  wbf[i] = __float2bfloat16_rn(p[i]);
-}
-
 __global__ void to_bf16_kernel(const float *__restrict__ p, __nv_bfloat16 *__restrict__ w, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) w[i] = __float2bfloat16_rn(p[i]);
-}
-
-__global__ void loss_sum_kernel(const float *__restrict__ l, int n, float *__restrict__ out) {
-  __shared__ float s[256];
-  float a = 0.f;
-  for (int i = threadIdx.x; i < n; i += 256) a += l[i];
-  s[threadIdx.x] = a;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[0] = s[0] / (float)n;
 }
 
 // ---------------------------------------------------------------------------
@@ -1103,45 +1243,33 @@ int mlp_upload_bf16(ct2g_ctx *ctx) {
   return CT2G_OK;
 }
 
-int stash_alloc(ct2g_ctx *ctx, size_t batch) {
-  ct2g_learn *L = ctx->learn;
-  if (L->stash_cap >= batch) return CT2G_OK;
-  if (L->stash) cudaFree(L->stash);
-  if (L->sloss) cudaFree(L->sloss);
-  L->stash = nullptr;
-  L->sloss = nullptr;
-  L->stash_cap = 0;
-  CT2G_CUDA(ctx, cudaMalloc(&L->stash, sizeof(float) * kStash * batch));
-  CT2G_CUDA(ctx, cudaMalloc(&L->sloss, sizeof(float) * (batch + 1)));
-  L->stash_cap = batch;
-  return CT2G_OK;
+// blocks of a gradient: one per tile of samples up to the two per SM that are
+// resident together (82 KB of shared memory each)
+int grad_blocks(const ct2g_ctx *ctx, int count) {
+  return std::max(1, std::min((count + TS - 1) / TS, 2 * ctx->num_sms));
 }
 
-// one optimisation batch (or, with lr == 0, only the gradient)
+// one optimisation batch (or, with lr == 0, only the gradient); grad[NP] gets
+// the loss
 int mlp_batch(ct2g_ctx *ctx, const float *X, const float *T, const uint32_t *idx, size_t start,
-              int count, float lr, float *loss_dev) {
+              int count, float lr) {
   ct2g_learn *L = ctx->learn;
   cudaStream_t st = ctx->stream;
-  const size_t smem = sizeof(float) * NP;
-  CT2G_TRY(ct2g_smem_attrs(ctx, mlp_fwdbwd_kernel, smem));
-  mlp_fwdbwd_kernel<<<ct2g_div_up(count, 128), 128, smem, st>>>(
-      L->wbf, L->fmean, L->fstd, X, T, idx, start, count, L->stash, L->sloss);
+  if (!L->gpart)
+    CT2G_CUDA(ctx, cudaMalloc(&L->gpart, sizeof(float) * NPL * 2 * (size_t)ctx->num_sms));
+  CT2G_TRY(ct2g_smem_attrs(ctx, mlp_grad_kernel, sizeof(GradSmem)));
+  const int nblk = grad_blocks(ctx, count);
+  mlp_grad_kernel<<<nblk, 256, sizeof(GradSmem), st>>>(L->wbf, L->fmean, L->fstd, X, T, idx,
+                                                       start, count, L->gpart);
   CT2G_LAUNCHED(ctx);
-  mlp_wgrad_kernel<<<ct2g_div_up(NP, 128), 128, 0, st>>>(L->fmean, L->fstd, X, idx, start, count,
-                                                          L->stash, L->grad);
-  CT2G_LAUNCHED(ctx);
-  if (loss_dev) {
-    loss_sum_kernel<<<1, 256, 0, st>>>(L->sloss, count, loss_dev);
-    CT2G_LAUNCHED(ctx);
-  }
+  AdamArgs adam{L->params, L->am, L->av, L->wbf, lr, 1.f, 1.f};
   if (lr > 0.f) {
     L->adam_t++;
-    const float c1 = 1.f - std::pow(0.9f, (float)L->adam_t);
-    const float c2 = 1.f - std::pow(0.999f, (float)L->adam_t);
-    adam_kernel<<<ct2g_div_up(NP, 256), 256, 0, st>>>(L->params, L->grad, L->am, L->av, L->wbf,
-                                                      lr, c1, c2);
-    CT2G_LAUNCHED(ctx);
+    adam.c1 = 1.f - std::pow(0.9f, (float)L->adam_t);
+    adam.c2 = 1.f - std::pow(0.999f, (float)L->adam_t);
   }
+  mlp_reduce_kernel<<<ct2g_div_up(NPL, 32), 256, 0, st>>>(L->gpart, nblk, count, L->grad, adam);
+  CT2G_LAUNCHED(ctx);
   return CT2G_OK;
 }
 
@@ -1161,7 +1289,7 @@ void ct2g_learned_free(ct2g_ctx *ctx) {
   if (!L) return;
   free_learn_cells(L);
   void *ptrs[] = {L->d_shell, L->d_shellG, L->d_stm, L->idx, L->d_cnt, L->params, L->grad, L->am, L->av, L->wbf,
-                  L->fmean, L->fstd, L->tX, L->tT, L->stash, L->sloss, L->tidx};
+                  L->fmean, L->fstd, L->tX, L->tT, L->gpart, L->gX, L->gT, L->tidx};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   delete L;
@@ -1195,7 +1323,7 @@ int ct2g_learned_enable(ct2g_ctx *ctx, float bwidth_ext) {
     CT2G_CUDA(ctx, cudaMalloc(&L->d_cnt, sizeof(uint32_t) * 8));
     CT2G_CUDA(ctx, cudaMemset(L->d_cnt, 0, sizeof(uint32_t) * 8));
     CT2G_CUDA(ctx, cudaMalloc(&L->params, sizeof(float) * NP));
-    CT2G_CUDA(ctx, cudaMalloc(&L->grad, sizeof(float) * NP));
+    CT2G_CUDA(ctx, cudaMalloc(&L->grad, sizeof(float) * NPL));
     CT2G_CUDA(ctx, cudaMalloc(&L->am, sizeof(float) * NP));
     CT2G_CUDA(ctx, cudaMalloc(&L->av, sizeof(float) * NP));
     CT2G_CUDA(ctx, cudaMalloc(&L->wbf, sizeof(__nv_bfloat16) * NP));
@@ -1443,11 +1571,9 @@ int ct2g_mlp_train(ct2g_ctx *ctx, int epochs, int batch, float lr, uint64_t seed
     norm_stats_kernel<<<NIN, 256, 0, st>>>(L->tX, L->tn, L->fmean, L->fstd);
     CT2G_LAUNCHED(ctx);
   }
-  CT2G_TRY(stash_alloc(ctx, (size_t)batch));
   std::vector<uint32_t> idx(L->tn);
   for (size_t i = 0; i < L->tn; i++) idx[i] = (uint32_t)i;
   std::mt19937_64 rng(seed);
-  float *dloss = L->sloss + batch;  // spare slot past the per-sample losses
   float last = 0.f;
   for (int e = 0; e < epochs; e++) {
     std::shuffle(idx.begin(), idx.end(), rng);
@@ -1455,7 +1581,7 @@ int ct2g_mlp_train(ct2g_ctx *ctx, int epochs, int batch, float lr, uint64_t seed
                                    cudaMemcpyHostToDevice, st));
     for (size_t s = 0; s < L->tn; s += (size_t)batch) {
       const int cnt = (int)std::min<size_t>(batch, L->tn - s);
-      CT2G_TRY(mlp_batch(ctx, L->tX, L->tT, L->tidx, s, cnt, lr, nullptr));
+      CT2G_TRY(mlp_batch(ctx, L->tX, L->tT, L->tidx, s, cnt, lr));
     }
     CT2G_CUDA(ctx, cudaStreamSynchronize(st));  // idx is reused next epoch
   }
@@ -1465,9 +1591,9 @@ int ct2g_mlp_train(ct2g_ctx *ctx, int epochs, int batch, float lr, uint64_t seed
   CT2G_CUDA(ctx, cudaMemcpyAsync(L->tidx, idx.data(), sizeof(uint32_t) * L->tn, cudaMemcpyHostToDevice, st));
   for (size_t s = 0; s < L->tn; s += (size_t)batch) {
     const int cnt = (int)std::min<size_t>(batch, L->tn - s);
-    CT2G_TRY(mlp_batch(ctx, L->tX, L->tT, L->tidx, s, cnt, 0.f, dloss));
+    CT2G_TRY(mlp_batch(ctx, L->tX, L->tT, L->tidx, s, cnt, 0.f));
     float h = 0.f;
-    CT2G_CUDA(ctx, cudaMemcpyAsync(&h, dloss, sizeof(float), cudaMemcpyDeviceToHost, st));
+    CT2G_CUDA(ctx, cudaMemcpyAsync(&h, L->grad + NP, sizeof(float), cudaMemcpyDeviceToHost, st));
     CT2G_CUDA(ctx, cudaStreamSynchronize(st));
     acc += (double)h * cnt;
   }
@@ -1483,31 +1609,31 @@ int ct2g_mlp_gradients(ct2g_ctx *ctx, const float *X, const float *T, size_t n, 
   if (!L) return CT2G_ESTATE;
   if (!L->have_mlp) return ct2g_fail(ctx, CT2G_ESTATE, "no MLP weights");
   if (!X || !T || !grad || n == 0 || n > (1u << 20)) return ct2g_fail(ctx, CT2G_EINVAL, "bad gradient arguments");
-  CT2G_TRY(stash_alloc(ctx, n));
-  float *dX = nullptr, *dT = nullptr;
-  uint32_t *dI = nullptr;
-  std::vector<uint32_t> idx(n);
-  for (size_t i = 0; i < n; i++) idx[i] = (uint32_t)i;
-  int rc = CT2G_OK;
-  cudaError_t e = cudaMalloc(&dX, sizeof(float) * NIN * n);
-  if (e == cudaSuccess) e = cudaMalloc(&dT, sizeof(float) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&dI, sizeof(uint32_t) * n);
-  if (e == cudaSuccess) e = cudaMemcpy(dX, X, sizeof(float) * NIN * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(dT, T, sizeof(float) * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(dI, idx.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) rc = ct2g_cuda_fail(ctx, e, "gradient inputs");
-  if (rc == CT2G_OK) rc = mlp_batch(ctx, dX, dT, dI, 0, (int)n, 0.f, L->sloss + n);
-  if (rc == CT2G_OK) {
-    e = cudaMemcpyAsync(grad, L->grad, sizeof(float) * NP, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess && loss)
-      e = cudaMemcpyAsync(loss, L->sloss + n, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) rc = ct2g_cuda_fail(ctx, e, "gradient outputs");
+  cudaStream_t st = ctx->stream;
+  if (L->g_cap < n) {
+    if (L->gX) cudaFree(L->gX);
+    if (L->gT) cudaFree(L->gT);
+    L->gX = L->gT = nullptr;
+    L->g_cap = 0;
+    CT2G_CUDA(ctx, cudaMalloc(&L->gX, sizeof(float) * NIN * n));
+    CT2G_CUDA(ctx, cudaMalloc(&L->gT, sizeof(float) * n));
+    L->g_cap = n;
   }
-  cudaStreamSynchronize(ctx->stream);
-  if (dX) cudaFree(dX);
-  if (dT) cudaFree(dT);
-  if (dI) cudaFree(dI);
+  int rc = CT2G_OK;
+  cudaError_t e = cudaMemcpyAsync(L->gX, X, sizeof(float) * NIN * n, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(L->gT, T, sizeof(float) * n, cudaMemcpyHostToDevice, st);
+  if (e != cudaSuccess) rc = ct2g_cuda_fail(ctx, e, "gradient inputs");
+  if (rc == CT2G_OK) rc = mlp_batch(ctx, L->gX, L->gT, nullptr, 0, (int)n, 0.f);
+  float last[NPL - NP];
+  if (rc == CT2G_OK) {
+    e = cudaMemcpyAsync(grad, L->grad, sizeof(float) * NP, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(last, L->grad + NP, sizeof(last), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) rc = ct2g_cuda_fail(ctx, e, "gradient outputs");
+    else if (loss) *loss = last[0];
+  }
+  cudaStreamSynchronize(st);  // the caller's arrays are free again on every return
   return rc;
 }
 

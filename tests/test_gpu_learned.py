@@ -114,6 +114,34 @@ def test_features_match_oracle(gpu):
     np.testing.assert_allclose(c["score"], score, rtol=1e-3, atol=1e-9)
 
 
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 130, 296 * 64 + 1])
+def test_mlp_gradient_tiles(gpu, n):
+    """Sample counts at the edges of the gradient kernel's 64-sample tiles and of
+    its resident blocks.  FP32 sums of n terms: within 1e-4 of the largest
+    gradient of each layer (n eps = 1e-3 at worst, sqrt(n) eps on average)."""
+    rng = np.random.default_rng(n)
+    params = (0.3 * rng.normal(size=OL.NP)).astype(np.float32)
+    fmean = rng.normal(size=OL.NIN).astype(np.float32)
+    fstd = rng.uniform(0.5, 2.0, OL.NIN).astype(np.float32)
+    X = rng.normal(size=(n, OL.NIN)).astype(np.float32)
+    T = rng.normal(size=n).astype(np.float32)
+    g = Gravity(mesh=16, order=2, bwidth=1.0, hsoft=1e-3)
+    g.learned_enable(2.0)
+    g.mlp_set(params, fmean, fstd)
+    grad, loss = g.mlp_gradients(X, T)
+    again, _ = g.mlp_gradients(X, T)
+    g.close()
+    loss_ref, grad_ref = OL.mlp_loss_grad(params, fmean, fstd, X, T)
+    assert np.array_equal(grad, again)  # a fixed order of summation
+    assert abs(loss - loss_ref) <= 1e-5 * loss_ref
+    for lo, hi in ((0, OL.OB1), (OL.OB1, OL.OW2), (OL.OW2, OL.OB2), (OL.OB2, OL.OW3),
+                   (OL.OW3, OL.OB3), (OL.OB3, OL.NP)):
+        gr = grad_ref[lo:hi]
+        # (the output bias' gradient is the mean error, which may cancel)
+        scale = max(np.abs(gr).max(), 2 * np.sqrt(loss_ref) if lo == OL.OB3 else 0.0)
+        assert np.abs(grad[lo:hi] - gr).max() <= 1e-4 * scale
+
+
 def test_mlp_gradients_match_oracle(gpu):
     _, g, _, _ = _setup(n=2000)
     g.mlp_init(seed=7)
