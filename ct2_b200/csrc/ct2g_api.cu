@@ -7,7 +7,6 @@
 
 #include "ct2g_internal.cuh"
 
-int ct2g_upload_stencil(ct2g_ctx *ctx, const std::vector<int> &st4);
 int ct2g_fft_init(ct2g_ctx *ctx);
 
 int ct2g_fail(ct2g_ctx *ctx, int code, const std::string &msg) {
@@ -377,21 +376,8 @@ int ct2g_create_boxes(const ct2g_options *opt, int nbox, ct2g_ctx **out) {
     if ((rc = ct2g_alloc_mesh(ctx)) != CT2G_OK) break;
     if ((rc = ct2g_fft_init(ctx)) != CT2G_OK) break;
     // near-field stencil: integer offsets |o|^2 <= bwidth^2 (the fixed form
-    // of particle_cell_neighbors, src/particle.cpp:302-318)
-    std::vector<int> st;
-    const int B = (int)std::floor(opt->bwidth);
+    // of particle_cell_neighbors, src/particle.cpp:302-318), as bit masks
     const double bw2 = (double)opt->bwidth * (double)opt->bwidth;
-    for (int i = -B; i <= B; i++)
-      for (int j = -B; j <= B; j++)
-        for (int k = -B; k <= B; k++)
-          if ((double)(i * i + j * j + k * k) <= bw2) {
-            st.push_back(i);
-            st.push_back(j);
-            st.push_back(k);
-            st.push_back(0);
-          }
-    ctx->nstencil = (int)(st.size() / 4);
-    if ((rc = ct2g_upload_stencil(ctx, st)) != CT2G_OK) break;
     // stencil bits per (in-block Morton position p, block offset (dX,dY,dZ)):
     // cells b of the neighbouring 4x4x4 block with |4 d + pos(b) - pos(p)|^2 <= bwidth^2
     {

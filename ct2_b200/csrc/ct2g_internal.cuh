@@ -325,9 +325,6 @@ struct ct2g_ctx {
   float2 *tw32 = nullptr;   // twiddles exp(-2 pi i k/M), k < M/2
   double2 *tw64 = nullptr;
   int tw_n = 0;
-  // stencil
-  int nstencil = 0;
-  int *d_stencil = nullptr;  // [nstencil][3]
 
   // state
   size_t rung_begin = 0;

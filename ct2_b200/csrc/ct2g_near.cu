@@ -18,8 +18,6 @@
 
 namespace {
 
-__constant__ int c_stencil[4 * 729];  // (ox, oy, oz, unused) per offset
-
 // ---------------------------------------------------------------------------
 // Near-field neighbour walk.  The stencil (offsets |o|^2 <= bwidth^2, bwidth
 // <= 4) of a cell touches the 27 4x4x4 cell blocks around its own; a block
@@ -29,21 +27,21 @@ __constant__ int c_stencil[4 * 729];  // (ox, oy, oz, unused) per offset
 // stencil cells.  Neighbour block keys come from dilated (bit-interleaved)
 // addition, which wraps periodically by itself.
 // ---------------------------------------------------------------------------
-__constant__ uint32_t c_doff[27 * 3];  // dilated block offsets, x/y/z lanes of the key
-
 struct Walk {
   uint32_t mx, my, mz;  // block-key masks of the x, y, z bits; the bits above
                         // them are the box index, which the walk keeps
+  // neighbouring block o = 9 (dx + 1) + 3 (dy + 1) + (dz + 1): a dilated step
+  // of -1 is every bit of the axis' mask, +1 its lowest bit (from the masks
+  // of this launch's own mesh: contexts of several meshes share the GPU)
+  __device__ __forceinline__ static uint32_t step(uint32_t sb, uint32_t m, int d) {
+    const uint32_t off = d == 0 ? m : d == 2 ? (m & (0u - m)) : 0u;
+    return ((sb | ~m) + off) & m;
+  }
   __device__ __forceinline__ uint32_t add(uint32_t sb, int o) const {
-    const uint32_t x = ((sb | ~mx) + c_doff[3 * o]) & mx;
-    const uint32_t y = ((sb | ~my) + c_doff[3 * o + 1]) & my;
-    const uint32_t z = ((sb | ~mz) + c_doff[3 * o + 2]) & mz;
-    return x | y | z | (sb & ~(mx | my | mz));
+    return step(sb, mx, o / 9) | step(sb, my, (o / 3) % 3) | step(sb, mz, o % 3) |
+           (sb & ~(mx | my | mz));
   }
 };
-
-// minimum-image offset (in cells) from cell c to cell n along one axis
-__device__ __forceinline__ int wrap_off(int n, int c, int M) { return ((n - c + M / 2) & (M - 1)) - M / 2; }
 
 // Near field, one warp per chunk of <= 32 sinks; the grid is persistent and
 // warps take chunks from a device work counter until the device-held chunk
@@ -846,24 +844,6 @@ int ct2g_near_dense_window(ct2g_ctx *ctx, const uint2 *chunks, const uint32_t *n
              : launch_near1<CT2G_SOFT_PLUMMER, false, false>(ctx, walk, chunks, nch, nullptr,
                                                              work, nullptr, stm, -1.f, 0.f, fx, fy,
                                                              fz, po, nullptr);
-}
-
-int ct2g_upload_stencil(ct2g_ctx *ctx, const std::vector<int> &st4) {
-  CT2G_CUDA(ctx, cudaMemcpyToSymbolAsync(c_stencil, st4.data(), sizeof(int) * st4.size(), 0,
-                                         cudaMemcpyHostToDevice, ctx->stream));
-  // dilated block offsets for the 27 neighbouring 4x4x4 blocks
-  const int nb = ctx->mbits - 2;
-  uint32_t d[27 * 3];
-  for (int o = 0; o < 27; o++) {
-    const int dd[3] = {o / 9 - 1, (o / 3) % 3 - 1, o % 3 - 1};
-    for (int a = 0; a < 3; a++) {
-      const uint32_t v = (uint32_t)dd[a] & ((1u << nb) - 1u);
-      d[3 * o + a] = ct2g_spread3(v) << (2 - a);
-    }
-  }
-  CT2G_CUDA(ctx, cudaMemcpyToSymbolAsync(c_doff, d, sizeof(d), 0, cudaMemcpyHostToDevice,
-                                         ctx->stream));
-  return CT2G_OK;
 }
 
 int ct2g_forces(ct2g_ctx *ctx, bool pot) {
