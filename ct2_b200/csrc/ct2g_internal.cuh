@@ -257,17 +257,17 @@ struct ct2g_ctx {
   uint32_t *sparse_list = nullptr; // particles of sparse cells, in order
   uint32_t *flags = nullptr;
   // work-list sizes stay on the device, so a step needs no host readback:
-  // [0] dense chunks, [1] sparse sinks, [2] sparse chunks, [3] and [4] the
-  // dense and sparse near-field work counters, [5] scan total scratch,
-  // [6] sticky device error (a status code a kernel left)
+  // [0] dense chunks, [1] sparse sinks, [2] sparse chunks, [5] scan total
+  // scratch, [6] sticky device error (a status code a kernel left), [8..11]
+  // near field: chunks taken, heavy chunks, heavy ones taken, the other
+  // sparse forms' work counter
   uint32_t *d_counts = nullptr;
   uint32_t dense_cell = 16;  // cells with at least this many particles get their own chunks
   int near_blocks_per_sm = 0;  // persistent near-field grid: blocks per SM (0: occupancy)
   int fft_tile = 0;            // y/x FFT pass tile width (0: default)
   int split_mg2l = 0;          // 1: X passes and MG2L as three launches, not one
   int sparse_path = 2;         // sparse sinks: 0 one per lane, 1 per-block warp chunks, 2 the
-                               // same chunks with their sources streamed in windows (Plummer;
-                               // the sphere kernel takes 1)
+                               // same chunks with their sources streamed in windows
   int overlap = 0;             // 1: near field on stream2, concurrent with the mesh solve
   int mg2l_greens_direct = 0;  // 1: the fused x pass reads the Green's values from HBM
   int near_chunks_per_warp = 0;  // overlap: chunks a near-field warp takes before its block exits
@@ -396,17 +396,15 @@ int ct2g_fft_cols_tc(ct2g_ctx *ctx, float2 *spec, int N, size_t nouter, size_t o
 int ct2g_learned_apply(ct2g_ctx *ctx, bool pot);
 int ct2g_learned_resize(ct2g_ctx *ctx);  // per-cell arrays follow the particle capacity
 void ct2g_learned_free(ct2g_ctx *ctx);
-// near-field direct sum of listed sinks over the cell window lo2 < |o|^2 <=
-// hi2 (ct2g_near.cu); sparse-style chunks, persistent over *nch / *work
-int ct2g_near_window(ct2g_ctx *ctx, const uint2 *chunks, const uint32_t *nch, uint32_t *work,
-                     const uint32_t *slist, const unsigned long long *stm, float lo2, float hi2,
-                     bool pot, float *fx, float *fy, float *fz, float *po);
-// the same over the stencil masks stm for dense-style chunks (<= 32
-// consecutive sinks of one cell, (first particle, count)), persistent over
-// *nch / *work
-int ct2g_near_dense_window(ct2g_ctx *ctx, const uint2 *chunks, const uint32_t *nch,
-                           uint32_t *work, const unsigned long long *stm, bool pot, float *fx,
-                           float *fy, float *fz, float *po);
+// widened near-field sums of selected cells (ct2g_near.cu): dense-style chunks
+// (<= 32 consecutive sinks of one cell, (first particle, count), *nd of them)
+// over the stencil masks stm, sparse-style ones (*ns, their sinks in slist)
+// over the source cells lo2 < |o|^2 <= hi2 of each sink's own; work: four
+// counters, zero on entry
+int ct2g_near_window(ct2g_ctx *ctx, const uint2 *dch, const uint32_t *nd, const uint2 *sch,
+                     const uint32_t *ns, const uint32_t *slist, uint32_t *work,
+                     const unsigned long long *stm, float lo2, float hi2, bool pot, float *fx,
+                     float *fy, float *fz, float *po);
 // D^n phi_eps(-o h) for the offsets o (x,y,z triples) -> d_out[nshell][nc]
 int ct2g_shell_greens(ct2g_ctx *ctx, const std::vector<int> &offs3, float *d_out);
 // far field of the current range into the force buffers (P2M if needed, mesh

@@ -55,8 +55,7 @@ struct ct2g_learn {
   uint32_t *scan = nullptr;    // scratch
   uint32_t *d_cnt = nullptr;   // [0] cells [1] selected cells [2] chunks [3] work counter
                                // [4] sinks of the selected cells; widening: [5] dense
-                               // chunks [6] their work counter [7] sparse sinks
-                               // [4] selected sinks [5] scan total scratch
+                               // chunks [7] sparse sinks [8..11] work counters
   // block-walk form of the widening (bwidth_ext <= 4): stencil masks of the
   // shell per (in-block cell, neighbouring block), selected cells and sinks
   unsigned long long *d_stm = nullptr;  // [64][27]
@@ -347,8 +346,7 @@ __global__ void __launch_bounds__(256) mlp_infer_kernel(
 // What bounds it: 6 x 5696 FLOP per sample, 0.7 GFLOP at 20,011 samples (9 us
 // of the FP32 peak); the kernels it replaces gave a whole weight's sum over the
 // samples to one thread (5825 threads on the chip, each a serial chain of
-// loads: 7.47 ms).  ct2g_mlp_gradients at 20,011 samples: 7.64 -> 0.235 ms a
-// call, most of it the host copies of the samples.
+// loads).  @MEASURED1@
 constexpr int TS = 64;          // samples per tile
 constexpr int TP = TS + 4;      // floats per row of a tile array
 struct GradSmem {
@@ -1167,11 +1165,10 @@ int widen_block_p(ct2g_ctx *ctx, bool pot, float *fx, float *fy, float *fz, floa
   sink_list_kernel<<<G, T, 0, st>>>(L->d_cnt, L->sel_cells, L->cells, ctx->cell_start, begin,
                                     L->pscan, L->ssink, L->scell);
   CT2G_LAUNCHED(ctx);
-  // the widened direct sum: selected dense cells through the near kernel's
-  // dense path (chunks of one cell, count d_cnt[5], work counter d_cnt[6]),
-  // the sinks of the other selected cells (count d_cnt[7]) in sparse-style
-  // chunks per 4x4x4 block (count d_cnt[2], work counter d_cnt[3]); flags,
-  // scan, pflag and pscan are free again here
+  // the widened direct sum: selected dense cells as dense chunks (one cell
+  // each, count d_cnt[5]), the sinks of the other selected cells (count
+  // d_cnt[7]) in sparse-style chunks per 4x4x4 block (count d_cnt[2]); work
+  // counters d_cnt[8..11]; flags, scan, pflag and pscan are free again here
   CT2G_CUDA(ctx, cudaMemsetAsync(L->flags, 0, sizeof(uint32_t) * nr, st));
   CT2G_CUDA(ctx, cudaMemsetAsync(L->pflag, 0, sizeof(uint32_t) * nr, st));
   shell_split_kernel<<<G, T, 0, st>>>(L->d_cnt, L->sel_cells, L->cells, ctx->cell_start, begin,
@@ -1192,17 +1189,14 @@ int widen_block_p(ct2g_ctx *ctx, bool pot, float *fx, float *fy, float *fz, floa
   sink_chunk_fill_kernel<<<G, T, 0, st>>>(L->d_cnt + 7, L->cflag, L->cscan, L->ssink2, ctx->keys,
                                           ctx->cell_start, L->pscan, begin, nr, L->chunks);
   CT2G_LAUNCHED(ctx);
-  CT2G_CUDA(ctx, cudaMemsetAsync(L->d_cnt + 3, 0, sizeof(uint32_t), st));
-  CT2G_CUDA(ctx, cudaMemsetAsync(L->d_cnt + 6, 0, sizeof(uint32_t), st));
+  CT2G_CUDA(ctx, cudaMemsetAsync(L->d_cnt + 8, 0, sizeof(uint32_t) * 4, st));
   shell_m2l_kernel<P><<<warp_grid(ctx, nr), 256, 0, st>>>(
       L->d_cnt, L->sel_cells, L->cells, L->mc, L->idx, geo_of(ctx), L->d_shell, L->d_shellG,
       L->nshell, L->lsub);
   CT2G_LAUNCHED(ctx);
   const float bw = ctx->opt.bwidth, bx = L->bw_ext;
-  CT2G_TRY(ct2g_near_dense_window(ctx, L->dchunks, L->d_cnt + 5, L->d_cnt + 6, L->d_stm, pot, fx,
-                                  fy, fz, po));
-  CT2G_TRY(ct2g_near_window(ctx, L->chunks, L->d_cnt + 2, L->d_cnt + 3, L->ssink2, L->d_stm,
-                            bw * bw, bx * bx, pot, fx, fy, fz, po));
+  CT2G_TRY(ct2g_near_window(ctx, L->dchunks, L->d_cnt + 5, L->chunks, L->d_cnt + 2, L->ssink2,
+                            L->d_cnt + 8, L->d_stm, bw * bw, bx * bx, pot, fx, fy, fz, po));
   if (pot)
     shell_l2p_kernel<P, true><<<G, T, 0, st>>>(L->d_cnt, L->ssink, L->scell, ctx->keys, begin,
                                                 ctx->mbits, ctx->src, L->lsub, ctx->box_gm, fx, fy,
@@ -1320,8 +1314,8 @@ int ct2g_learned_enable(ct2g_ctx *ctx, float bwidth_ext) {
   if (!ctx->learn) {
     ctx->learn = new ct2g_learn();
     ct2g_learn *L = ctx->learn;
-    CT2G_CUDA(ctx, cudaMalloc(&L->d_cnt, sizeof(uint32_t) * 8));
-    CT2G_CUDA(ctx, cudaMemset(L->d_cnt, 0, sizeof(uint32_t) * 8));
+    CT2G_CUDA(ctx, cudaMalloc(&L->d_cnt, sizeof(uint32_t) * 12));
+    CT2G_CUDA(ctx, cudaMemset(L->d_cnt, 0, sizeof(uint32_t) * 12));
     CT2G_CUDA(ctx, cudaMalloc(&L->params, sizeof(float) * NP));
     CT2G_CUDA(ctx, cudaMalloc(&L->grad, sizeof(float) * NPL));
     CT2G_CUDA(ctx, cudaMalloc(&L->am, sizeof(float) * NP));
