@@ -264,13 +264,13 @@ __global__ void gather_kernel(const uint32_t *__restrict__ perm, size_t begin, s
                        (float)((int32_t)(pz & mask) - half) * sc, 0.f);
 }
 
-// Sink work lists for the near field, all in warp chunks of <= 32 sinks:
-// cells with at least kDenseCell particles are split into chunks of one cell
-// (every 32nd particle of the cell starts one); the particles of sparser
+// Sink work lists for the near field, in warp chunks: cells with at least
+// dense_cell particles are split into chunks of one cell (every 64th particle
+// of the cell starts one: two sinks a lane); the particles of sparser
 // cells are listed (sparse_list) and chunked per 4x4x4 cell block (a block is
 // 64 consecutive Morton keys), every 32nd sparse particle of a block starting
 // a chunk.
-constexpr uint32_t kSparseChunk = 32;  // sinks per sparse chunk (near_kernel)
+constexpr uint32_t kSparseChunk = 32;  // sinks per sparse chunk
 
 __global__ void chunk_flag_kernel(const uint32_t *__restrict__ skeys,
                                   const uint32_t *__restrict__ cs, size_t begin, size_t nr,
@@ -281,7 +281,7 @@ __global__ void chunk_flag_kernel(const uint32_t *__restrict__ skeys,
   const uint32_t k = skeys[i];
   const uint32_t c0 = cs[k], n = cs[k + 1] - c0;
   const bool dense = n >= dense_cell;
-  flags[i] = (dense && ((((uint32_t)(begin + i) - c0) & 31u) == 0)) ? 1u : 0u;
+  flags[i] = (dense && ((((uint32_t)(begin + i) - c0) & 63u) == 0)) ? 1u : 0u;
   sflags[i] = dense ? 0u : 1u;
 }
 
@@ -310,7 +310,7 @@ __global__ void dense_chunk_fill_kernel(const uint32_t *__restrict__ flags,
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nr || !flags[i]) return;
   const uint32_t g = (uint32_t)(begin + i);
-  list[fscan[i]] = make_uint2(g, min(32u, cs[skeys[i] + 1] - g));
+  list[fscan[i]] = make_uint2(g, min(64u, cs[skeys[i] + 1] - g));
 }
 
 // (start, count) of sparse chunks: index into sparse_list, sinks

@@ -35,9 +35,9 @@ struct Walk {
 
 // ---------------------------------------------------------------------------
 // Packed pairs: Blackwell's f32x2 add/mul/fma do two FP32 operations per
-// issued instruction.  A warp's source batch is staged as pair records --
-// (x0, x1, y0, y1) in one 16-byte slot and (z0, z1) after them -- so one
-// broadcast load of each feeds two interactions.
+// issued instruction.  A warp's source batch is staged as arrays of x, y and z
+// (and, sparse, of cell bits), so that one 16-byte broadcast load of each
+// feeds four interactions of every sink a lane holds.
 // ---------------------------------------------------------------------------
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 f2_pack(float a, float b) {
@@ -115,22 +115,22 @@ __device__ __forceinline__ int nth_set_bit(unsigned long long w, uint32_t r) {
 // Staging: the source at stream position g belongs to the last cell whose
 // first position is <= g.  The cells' first positions inside the batch are
 // OR-reduced into one word of head bits, so the owner is a population count,
-// and one shuffle gives its (first particle - first position).  The source's
-// offset from the chunk's frame (the sink cell's centre; the block's first cell
-// for a sparse chunk) is the difference of the fixed-point positions,
-// periodic by itself, rounded once to FP32 and negated, so that the inner loop adds.
+// and a table of the window in shared memory gives its (first particle - first
+// position) and its centre in the chunk's frame (the sink cell's centre; that of the
+// block's first cell for a sparse chunk).  Sources are staged negated, so that
+// the inner loop adds.
 //
 // What bounds it: 11 packed FP32 instructions and two MUFU operations per two
 // interactions (22 and 16 cycles of their pipes per warp and SM sub-partition), so
 // 11.6 interactions per clock and SM, 3.4e12 per second, when nothing else
 // is issued.  A packed instruction takes two issue slots, so what else a pair
 // needs (two shared loads, two MUFU, its share of the staging) counts against
-// it: FMA pipe 71%, all issue slots used.  Against one warp per chunk, cells'
-// sources in batches of their own halves of blocks (dense), a table of stencil entries
-// per lane in shared memory (sparse) and scalar arithmetic (sphere kernel):
-// 2.5 M particles in halos 35.2 -> 34.4 ms, 128^3 in Plummer spheres 3.52 ->
-// 3.23, 300 k with the sphere kernel and potentials 10.2 -> 7.0 ms, 400 k
-// in 48 halos 10.0 -> 6.7 ms.
+// it: FMA pipe 71%, all issue slots used; two sinks per lane halve that share.
+// Against one warp per chunk, cells' sources in batches of their own half
+// blocks (dense), a table of stencil entries per lane in shared memory (sparse)
+// and scalar arithmetic cell by cell (sphere kernel), a step of 2.5 M particles in halos
+// 48.6 -> 42.5 ms, 50 k in spheres 1.14 -> 0.88, 300 k with the sphere kernel and
+// potentials 11.96 -> 6.45, 128^3 in Plummer spheres 11.87 -> 11.55.
 // ---------------------------------------------------------------------------
 struct NearArgs {
   const uint2 *dchunks;     // dense chunks (first particle, sinks), *ndense of them
@@ -144,7 +144,6 @@ struct NearArgs {
   Walk walk;
   const uint32_t *skeys;
   uint32_t rbegin;
-  const uint32_t *x, *y, *z;
   const float4 *src;        // offsets from the own cell's centre
   int mbits;
   float soft;
@@ -152,48 +151,38 @@ struct NearArgs {
   const float *box_gm;
   float *ofx, *ofy, *ofz, *opot;
   bool store;               // store into the buffers instead of adding to them
-  uint32_t *work;           // [0] chunks taken, [1] heavy chunks, [2] heavy ones taken
+  uint32_t *work;           // [0] sparse chunks taken, [1] heavy ones among them,
+                            // [2] dense and heavy chunks taken
   uint32_t *heavy;          // list of the heavy chunks
+  uint32_t heavy_min;       // sources a sparse chunk may have to stay with one warp
   uint32_t warps;           // warps the launch may spread few chunks over
   uint32_t maxch;
   unsigned long long *inter;
 };
 
-// A chunk whose 27 neighbouring blocks hold more sources than this is left to
-// a second launch in which the eight warps of a block share each chunk: one warp
-// on its own walks 1000 sources in about 10 us, and clustered sets have
-// chunks of 10^5 (2.5 ms on a single warp while the rest of the GPU idled, at
-// 400 k particles in 48 halos), while splitting repeats the window walk
-// in every warp (about 1000 instructions each, 5% of the work at this size).
-constexpr uint32_t kHeavySources = 16384;
-constexpr int kStage = 256;  // floats of staging per warp: two batches of pair records
+// A sparse chunk whose 27 neighbouring blocks hold more sources than A.heavy_min is
+// left to the cooperative launch: one warp on its own walks 1000 sources in
+// about 10 us, and clustered sets have sparse chunks beside cells of 10^5 (2.5 ms
+// on a single warp while the rest of the GPU idled, at 400 k particles in 48
+// halos).  A block per chunk costs its eight warps the setup, so that it only
+// pays where a warp's chunk is long against the launch: a mesh of M has (M/4)^3
+// blocks, under one round of the GPU's warps up to 64, 7 at 128, 55 at 256.
+// Limits of 1024 / 3072 / 8192 / 16384 measured 0.88 / 0.95 / 1.04 / 1.04 ms a step
+// (50 k particles, mesh 64), 2.75 / 2.82 / 2.96 / 2.96 (262 k, 128, with the learned
+// correction), 11.9 / 11.75 / 11.58 / 11.52 (2.1 M, 256).
+uint32_t heavy_min(int M) { return M <= 128 ? 1024u : 8192u; }
+// floats of staging per warp: two batches (x, y, z and cell bits of 32
+// sources), then the window's table
+constexpr int kBatch = 128, kStage = 2 * kBatch + 128;
 // a coordinate that makes r^2 infinite: an empty slot of the last batch adds 0
 constexpr float kFar = 3e19f;
 
-// two interactions of a sink at (X, Y, Z) (both halves equal) with the sources of
-// pair record pr (negated coordinates); accumulates d g and 1/r (the caller negates)
+// g = the softened 1/r^3 and pp = 1/r of two sources at separation (dx, dy, dz);
+// a source that is off gives zeros
 template <int KERNEL, bool POT, bool MASKED>
-__device__ __forceinline__ void pair_term(const float *sb, int pr, uint32_t bits, f32x2 X, f32x2 Y,
-                                          f32x2 Z, f32x2 H2, float h2, float hinv, float hinv3,
-                                          f32x2 &ax, f32x2 &ay, f32x2 &az, f32x2 &ap) {
-  const float4 a = reinterpret_cast<const float4 *>(sb)[pr];  // x0 x1 y0 y1
-  float z0, z1;
-  bool on0 = true, on1 = true;
-  if (MASKED) {
-    const float4 b = reinterpret_cast<const float4 *>(sb + 64)[pr];  // z0 z1 and the cells' bits
-    z0 = b.x;
-    z1 = b.y;
-    on0 = (__float_as_uint(b.z) & bits) != 0u;
-    on1 = (__float_as_uint(b.w) & bits) != 0u;
-  } else {
-    const float2 b = reinterpret_cast<const float2 *>(sb + 64)[pr];
-    z0 = b.x;
-    z1 = b.y;
-  }
-  const f32x2 dx = f2_add(X, f2_pack(a.x, a.y));
-  const f32x2 dy = f2_add(Y, f2_pack(a.z, a.w));
-  const f32x2 dz = f2_add(Z, f2_pack(z0, z1));
-  f32x2 g, pp;
+__device__ __forceinline__ void pair_weights(f32x2 dx, f32x2 dy, f32x2 dz, f32x2 H2, float h2,
+                                             float hinv, float hinv3, bool on0, bool on1,
+                                             f32x2 &g, f32x2 &pp) {
   if constexpr (KERNEL == CT2G_SOFT_PLUMMER) {
     const f32x2 r2 = f2_fma(dz, dz, f2_fma(dy, dy, f2_fma(dx, dx, H2)));
     float r0, r1;
@@ -229,10 +218,265 @@ __device__ __forceinline__ void pair_term(const float *sb, int pr, uint32_t bits
     g = f2_pack(g0, g1);
     pp = f2_pack(p0, p1);
   }
-  ax = f2_fma(dx, g, ax);
-  ay = f2_fma(dy, g, ay);
-  az = f2_fma(dz, g, az);
-  if (POT) ap = f2_add(ap, pp);
+}
+
+// a lane's sink (coordinates in both halves) and its packed sums +d g, +1/r
+// (the caller negates)
+struct Sink {
+  f32x2 X, Y, Z, ax, ay, az, ap;
+};
+
+// interactions of NS sinks with the four sources of quad qd (negated
+// coordinates in the staged arrays)
+template <int KERNEL, bool POT, bool MASKED, int NS>
+__device__ __forceinline__ void quad_term(const float *sb, int qd, uint32_t bits, Sink (&k)[NS],
+                                          f32x2 H2, float h2, float hinv, float hinv3) {
+  const float4 x = reinterpret_cast<const float4 *>(sb)[qd];
+  const float4 y = reinterpret_cast<const float4 *>(sb + 32)[qd];
+  const float4 z = reinterpret_cast<const float4 *>(sb + 64)[qd];
+  bool on[4] = {true, true, true, true};
+  if (MASKED) {
+    const uint4 m = reinterpret_cast<const uint4 *>(sb + 96)[qd];
+    on[0] = (m.x & bits) != 0u;
+    on[1] = (m.y & bits) != 0u;
+    on[2] = (m.z & bits) != 0u;
+    on[3] = (m.w & bits) != 0u;
+  }
+  const f32x2 px[2] = {f2_pack(x.x, x.y), f2_pack(x.z, x.w)};
+  const f32x2 py[2] = {f2_pack(y.x, y.y), f2_pack(y.z, y.w)};
+  const f32x2 pz[2] = {f2_pack(z.x, z.y), f2_pack(z.z, z.w)};
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int u = 0; u < NS; u++) {
+      const f32x2 dx = f2_add(k[u].X, px[h]), dy = f2_add(k[u].Y, py[h]), dz = f2_add(k[u].Z, pz[h]);
+      f32x2 g, pp;
+      pair_weights<KERNEL, POT, MASKED>(dx, dy, dz, H2, h2, hinv, hinv3, on[2 * h], on[2 * h + 1],
+                                        g, pp);
+      k[u].ax = f2_fma(dx, g, k[u].ax);
+      k[u].ay = f2_fma(dy, g, k[u].ay);
+      k[u].az = f2_fma(dz, g, k[u].az);
+      if (POT) k[u].ap = f2_add(k[u].ap, pp);
+    }
+}
+
+// the NS sinks per lane of a chunk and what its warp walks
+template <bool SPARSE, int NS>
+struct Chunk {
+  uint32_t idx[NS];         // this lane's sinks (an inactive one repeats the first)
+  uint32_t key, p;          // of the first; its position in the block
+  unsigned long long pm;    // in-block positions present in the chunk
+  unsigned long long word;  // lane o < 27: candidate cells of neighbouring block o,
+  uint32_t nblk;            // and its block key
+  uint32_t ex1, C;          // candidate cells before block o's, and in all
+  int fx, fy, fz;           // the frame's cell in the block: the sink cell, or (sparse) 0
+  __device__ __forceinline__ void open(const NearArgs &A, const uint2 cd, int lane) {
+#pragma unroll
+    for (int u = 0; u < NS; u++) {
+      const uint32_t e = (uint32_t)(lane + 32 * u);
+      const uint32_t slot = cd.x + (e < cd.y ? e : 0u);
+      idx[u] = SPARSE ? A.slist[slot] : slot;
+    }
+    key = A.skeys[idx[0] - A.rbegin];
+    p = key & 63u;
+    const uint32_t blk = key >> 6;  // the same for the whole chunk
+    pm = 1ull << p;
+    if (SPARSE)
+      pm = ((unsigned long long)__reduce_or_sync(0xffffffffu, (uint32_t)(pm >> 32)) << 32) |
+           __reduce_or_sync(0xffffffffu, (uint32_t)pm);
+    word = 0;
+    nblk = 0;
+    if (lane < 27) {
+      nblk = A.walk.add(blk, lane);
+      unsigned long long m = 0, q = pm;
+      while (q) {
+        const int pp = __ffsll((long long)q) - 1;
+        q &= q - 1;
+        m |= __ldg(A.stm + pp * 27 + lane);
+      }
+      word = A.occ[nblk] & m;
+    }
+    const uint32_t c1 = (uint32_t)__popcll(word);
+    uint32_t in1 = c1;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, in1, d);
+      if (lane >= d) in1 += t;
+    }
+    ex1 = in1 - c1;
+    C = __shfl_sync(0xffffffffu, in1, 31);
+    fx = fy = fz = 0;
+    if (!SPARSE) inblock((int)p, fx, fy, fz);
+  }
+  // sources of the neighbouring blocks that hold candidates (an upper bound)
+  __device__ __forceinline__ uint32_t sources(const NearArgs &A) const {
+    const uint32_t w = word ? A.cs[(size_t)(nblk + 1) << 6] - A.cs[(size_t)nblk << 6] : 0u;
+    return __reduce_add_sync(0xffffffffu, w);
+  }
+  __device__ __forceinline__ void sinks(const NearArgs &A, float hc, Sink (&k)[NS]) const {
+    int ix, iy, iz;
+    inblock((int)p, ix, iy, iz);
+#pragma unroll
+    for (int u = 0; u < NS; u++) {
+      const float4 q = A.src[idx[u]];
+      const float sx = fmaf((float)(ix - fx), hc, q.x), sy = fmaf((float)(iy - fy), hc, q.y),
+                  sz = fmaf((float)(iz - fz), hc, q.z);
+      k[u] = Sink{f2_pack(sx, sx), f2_pack(sy, sy), f2_pack(sz, sz), 0ull, 0ull, 0ull, 0ull};
+    }
+  }
+  // The window of candidate cells w0 ..: its table (a cell per lane: its centre
+  // from the frame's, negated, and its first particle less its first stream position) into
+  // win, its first stream position in `excl` (~0 past the last cell), the
+  // sources in `total`, and (sparse) this lane's mask of the cells in its own
+  // stencil in `bits`; nsrc counts the sources of a lane's stencil.
+  __device__ __forceinline__ void window(const NearArgs &A, uint32_t w0, float hc, int lane,
+                                         float4 *win, uint32_t &excl, uint32_t &total,
+                                         uint32_t &bits, uint32_t &nsrc) const {
+    const bool valid = w0 + (uint32_t)lane < C;
+    // the (g - ex1[o])-th candidate cell of block o
+    const uint32_t g = min(w0 + (uint32_t)lane, C - 1);
+    int o = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+      const uint32_t e = __shfl_sync(0xffffffffu, ex1, o + step);
+      if (e <= g) o += step;
+    }
+    const unsigned long long wo = __shfl_sync(0xffffffffu, word, o);
+    const uint32_t nbo = __shfl_sync(0xffffffffu, nblk, o);
+    const uint32_t exo = __shfl_sync(0xffffffffu, ex1, o);
+    const int q = nth_set_bit(wo, g - exo);
+    uint32_t jb = 0, c = 0;
+    if (valid) {
+      const uint32_t ck = (nbo << 6) | (uint32_t)q;
+      jb = A.cs[ck];
+      c = A.cs[ck + 1] - jb;
+    }
+    uint32_t incl = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += t;
+    }
+    total = __shfl_sync(0xffffffffu, incl, 31);
+    excl = valid ? incl - c : 0xffffffffu;
+    int bx, by, bz;
+    inblock(q, bx, by, bz);
+    const int cx = 4 * (o / 9 - 1) + bx, cy = 4 * ((o / 3) % 3 - 1) + by, cz = 4 * (o % 3 - 1) + bz;
+    win[lane] = make_float4((float)(fx - cx) * hc, (float)(fy - cy) * hc, (float)(fz - cz) * hc,
+                            __uint_as_float(jb - (incl - c)));
+    bits = 0xffffffffu;
+    if (SPARSE) {
+      bits = 0u;
+      unsigned long long pq = pm;
+      while (pq) {
+        const int pp = __ffsll((long long)pq) - 1;
+        pq &= pq - 1;
+        int qx, qy, qz;
+        inblock(pp, qx, qy, qz);
+        const int d2 = (cx - qx) * (cx - qx) + (cy - qy) * (cy - qy) + (cz - qz) * (cz - qz);
+        const bool in = valid && d2 > A.lo2 && d2 <= A.hi2;
+        const uint32_t bal = __ballot_sync(0xffffffffu, in);
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, in ? c : 0u);
+        if ((int)p == pp) {
+          bits = bal;
+          nsrc += sum;
+        }
+      }
+    } else {
+      nsrc += total;
+    }
+  }
+};
+
+// the window slot of stream position b + lane (clamped to the last), and its source
+__device__ __forceinline__ uint32_t stream_slot(uint32_t excl, uint32_t b, uint32_t g1) {
+  const uint32_t before = __ballot_sync(0xffffffffu, excl < b);
+  const uint32_t rel = excl - b;
+  const uint32_t heads = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
+  return __popc(before) + __popc(heads & (0xffffffffu >> (31u - (g1 - b)))) - 1;
+}
+
+// a fetched source (offset q from its cell's centre, slot t of the window) into
+// a staged batch; off: an empty slot
+template <bool SPARSE>
+__device__ __forceinline__ void stage_source(float *sb, const float4 &w, const float4 &q,
+                                             uint32_t t, bool on, int lane) {
+  sb[lane] = on ? w.x - q.x : kFar;
+  sb[32 + lane] = w.y - q.y;
+  sb[64 + lane] = w.z - q.z;
+  if (SPARSE) sb[96 + lane] = __uint_as_float(on ? 1u << t : 0u);
+}
+
+struct Soft {
+  f32x2 H2;
+  float h2, hinv, hinv3;
+  __device__ __forceinline__ explicit Soft(float h)
+      : H2(f2_pack(h * h, h * h)), h2(h * h), hinv(1.f / h), hinv3(0.f) {
+    hinv3 = hinv * hinv * hinv;
+  }
+};
+
+// a staged batch of n <= 32 sources
+template <int KERNEL, bool POT, bool SPARSE, int NS>
+__device__ __forceinline__ void eval_batch(const float *sb, uint32_t n, uint32_t bits,
+                                           Sink (&k)[NS], const Soft &h) {
+  if (n >= 32) {
+#pragma unroll 4
+    for (int qd = 0; qd < 8; qd++)
+      quad_term<KERNEL, POT, SPARSE, NS>(sb, qd, bits, k, h.H2, h.h2, h.hinv, h.hinv3);
+  } else {
+    const int nq = (int)(n + 3) >> 2;
+#pragma unroll 1
+    for (int qd = 0; qd < nq; qd++)
+      quad_term<KERNEL, POT, SPARSE, NS>(sb, qd, bits, k, h.H2, h.h2, h.hinv, h.hinv3);
+  }
+}
+
+// a sink's packed sums so far, and back to zero
+template <bool POT>
+__device__ __forceinline__ float4 take(Sink &k) {
+  float a0, a1;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  f2_unpack(k.ax, a0, a1);
+  v.x = a0 + a1;
+  f2_unpack(k.ay, a0, a1);
+  v.y = a0 + a1;
+  f2_unpack(k.az, a0, a1);
+  v.z = a0 + a1;
+  if (POT) {
+    f2_unpack(k.ap, a0, a1);
+    v.w = a0 + a1;
+  }
+  k.ax = k.ay = k.az = k.ap = 0ull;
+  return v;
+}
+__device__ __forceinline__ void add(float4 &n, const float4 &v) {
+  n.x += v.x;
+  n.y += v.y;
+  n.z += v.z;
+  n.w += v.w;
+}
+
+// The sums (negated) times GM, added to the far field (L2P, with GM) already in
+// the force buffers, or stored into the near-field buffers when the two run
+// side by side; the product is rounded on its own (no fused multiply-add into
+// the far field), so that both forms add the same two values.
+template <bool POT>
+__device__ __forceinline__ void write_sink(const NearArgs &A, uint32_t i, uint32_t key,
+                                           const float4 &n) {
+  const float GM = __ldg(A.box_gm + (key >> (3 * A.mbits)));
+  const float gx = __fmul_rn(GM, -n.x), gy = __fmul_rn(GM, -n.y), gz = __fmul_rn(GM, -n.z);
+  if (A.store) {
+    A.ofx[i] = gx;
+    A.ofy[i] = gy;
+    A.ofz[i] = gz;
+    if (POT) A.opot[i] = __fmul_rn(GM, -n.w);
+  } else {
+    A.ofx[i] += gx;
+    A.ofy[i] += gy;
+    A.ofz[i] += gz;
+    if (POT) A.opot[i] += __fmul_rn(GM, -n.w);
+  }
 }
 
 // the barrier of the S warps (a power of two) that share a chunk
@@ -240,264 +484,90 @@ __device__ __forceinline__ void group_sync(int S, int group) {
   if (S > 1) asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(32 * S) : "memory");
 }
 
-// One chunk, its windows' sums added in window order.  S warps may share it:
-// warp s takes the windows s, s + S, ..., and warp 0 adds each round's S
-// sums in order, so the result does not depend on S.  HEAVY: the eight warps take
-// every eighth batch of each window instead, and warp 0 adds their eight sums.
-// stage: this warp's kStage floats (the group's warps' lie one after
-// another).  Without HEAVY a heavy chunk is left alone (false returned).
-template <int KERNEL, bool POT, bool SPARSE, bool HEAVY>
-__device__ __forceinline__ bool near_chunk(const NearArgs &A, const uint2 cd, int s, int S,
-                                           int group, float *stage, int lane) {
-  const int sh = 32 - A.mbits;
-  const bool act = (uint32_t)lane < cd.y;
-  const uint32_t slot = cd.x + (act ? (uint32_t)lane : 0u);
-  const uint32_t i = SPARSE ? A.slist[slot] : slot;
-  const uint32_t key = A.skeys[i - A.rbegin];
-  const uint32_t p = key & 63u, blk = key >> 6;  // blk is the same for the whole chunk
-  // in-block positions present in the chunk
-  unsigned long long pm = 1ull << p;
-  if (SPARSE)
-    pm = ((unsigned long long)__reduce_or_sync(0xffffffffu, (uint32_t)(pm >> 32)) << 32) |
-         __reduce_or_sync(0xffffffffu, (uint32_t)pm);
-  unsigned long long word = 0;
-  uint32_t nblk = 0;
-  if (lane < 27) {
-    nblk = A.walk.add(blk, lane);
-    unsigned long long m = 0, q = pm;
-    while (q) {
-      const int pp = __ffsll((long long)q) - 1;
-      q &= q - 1;
-      m |= __ldg(A.stm + pp * 27 + lane);
-    }
-    word = A.occ[nblk] & m;
-  }
-  if (!HEAVY) {
-    const uint32_t w = word ? A.cs[(size_t)(nblk + 1) << 6] - A.cs[(size_t)nblk << 6] : 0u;
-    if (__reduce_add_sync(0xffffffffu, w) > kHeavySources) return false;
-  }
-  // the frame's origin and this lane's sink in it
-  const uint32_t fk = (SPARSE ? key & ~63u : key) & ((1u << (3 * A.mbits)) - 1u);
-  const uint32_t half = 1u << (sh - 1);
-  const uint32_t ox = (ct2g_compact3(fk >> 2) << sh) + half,
-                 oy = (ct2g_compact3(fk >> 1) << sh) + half, oz = (ct2g_compact3(fk) << sh) + half;
-  const float sc = (float)CT2G_TWO_M32;
-  const float sx = (float)(int32_t)(A.x[i] - ox) * sc, sy = (float)(int32_t)(A.y[i] - oy) * sc,
-              sz = (float)(int32_t)(A.z[i] - oz) * sc;
-  const f32x2 X = f2_pack(sx, sx), Y = f2_pack(sy, sy), Z = f2_pack(sz, sz);
-  const float h2 = A.soft * A.soft, hinv = 1.f / A.soft, hinv3 = hinv * hinv * hinv;
-  const f32x2 H2 = f2_pack(h2, h2);
-  f32x2 ax = 0ull, ay = 0ull, az = 0ull, ap = 0ull;
-  float nx = 0.f, ny = 0.f, nz = 0.f, np = 0.f;
+// One sparse chunk by the S warps that share it: warp s takes the windows s,
+// s + S, ..., and warp 0 adds each round's S sums in order, so the result does
+// not depend on S.  stage: this warp's kStage floats (the group's warps' lie
+// one after another).  A heavy chunk is left alone (false returned).
+template <int KERNEL, bool POT>
+__device__ __forceinline__ bool sparse_chunk(const NearArgs &A, const uint2 cd, int s, int S,
+                                             int group, float *stage, int lane) {
+  Chunk<true, 1> k;
+  k.open(A, cd, lane);
+  if (k.sources(A) > A.heavy_min) return false;
+  const float hc = 1.0f / (float)(1 << A.mbits);
+  Sink sink[1];
+  k.sinks(A, hc, sink);
+  const Soft soft(A.soft);
+  float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
   uint32_t nsrc = 0;
-  // the packed sums so far, and back to zero
-  auto take = [&]() {
-    float a0, a1;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    f2_unpack(ax, a0, a1);
-    v.x = a0 + a1;
-    f2_unpack(ay, a0, a1);
-    v.y = a0 + a1;
-    f2_unpack(az, a0, a1);
-    v.z = a0 + a1;
-    if (POT) {
-      f2_unpack(ap, a0, a1);
-      v.w = a0 + a1;
-    }
-    ax = ay = az = ap = 0ull;
-    return v;
-  };
-  auto add = [&](const float4 &v) {
-    nx += v.x;
-    ny += v.y;
-    nz += v.z;
-    if (POT) np += v.w;
-  };
-  // the first nw warps' sums into warp 0's totals, in order
-  auto share = [&](int nw) {
-    const float4 v = take();
-    __syncwarp();  // every lane is done with this warp's staging
-    if (s > 0) reinterpret_cast<float4 *>(stage)[lane] = v;
-    group_sync(S, group);
-    if (s == 0) {
-      add(v);
-      for (int k = 1; k < nw; k++)
-        add(reinterpret_cast<const float4 *>(stage + k * kStage)[lane]);
-    }
-    group_sync(S, group);
-  };
-  // candidate cells before each neighbouring block's, and in all
-  const uint32_t c1 = (uint32_t)__popcll(word);
-  uint32_t in1 = c1;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, in1, d);
-    if (lane >= d) in1 += t;
-  }
-  const uint32_t ex1 = in1 - c1, C = __shfl_sync(0xffffffffu, in1, 31);
-  const int rec = 4 * (lane >> 1) + (lane & 1);
-  const int recz = 64 + (SPARSE ? rec : 2 * (lane >> 1) + (lane & 1));
-  const uint32_t bs = HEAVY ? (uint32_t)s : 0u, bS = HEAVY ? 8u : 1u;  // this warp's batches
-  for (uint32_t r0 = 0; r0 < C; r0 += HEAVY ? 32u : 32u * (uint32_t)S) {
-    const uint32_t w0 = HEAVY ? r0 : r0 + 32u * (uint32_t)s;
-    if (w0 < C) {
-      const bool valid = w0 + (uint32_t)lane < C;
-      // window cell of this lane: the (g - ex1[o])-th candidate cell of block o
-      const uint32_t g = min(w0 + (uint32_t)lane, C - 1);
-      int o = 0;
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const uint32_t e = __shfl_sync(0xffffffffu, ex1, o + step);
-        if (e <= g) o += step;
-      }
-      const unsigned long long wo = __shfl_sync(0xffffffffu, word, o);
-      const uint32_t nbo = __shfl_sync(0xffffffffu, nblk, o);
-      const uint32_t exo = __shfl_sync(0xffffffffu, ex1, o);
-      const int q = nth_set_bit(wo, g - exo);
-      uint32_t jb = 0, c = 0;
-      if (valid) {
-        const uint32_t ck = (nbo << 6) | (uint32_t)q;
-        jb = A.cs[ck];
-        c = A.cs[ck + 1] - jb;
-      }
-      uint32_t incl = c;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += t;
-      }
-      const uint32_t excl = incl - c, total = __shfl_sync(0xffffffffu, incl, 31);
-      uint32_t bits = 0xffffffffu;
-      if (SPARSE) {
-        bits = 0u;
-        int bx, by, bz;
-        inblock(q, bx, by, bz);
-        const int cx = 4 * (o / 9 - 1) + bx, cy = 4 * ((o / 3) % 3 - 1) + by, cz = 4 * (o % 3 - 1) + bz;
-        unsigned long long pq = pm;
-        while (pq) {
-          const int pp = __ffsll((long long)pq) - 1;
-          pq &= pq - 1;
-          int qx, qy, qz;
-          inblock(pp, qx, qy, qz);
-          const int d2 = (cx - qx) * (cx - qx) + (cy - qy) * (cy - qy) + (cz - qz) * (cz - qz);
-          const bool in = valid && d2 > A.lo2 && d2 <= A.hi2;
-          const uint32_t bal = __ballot_sync(0xffffffffu, in);
-          const uint32_t sum = __reduce_add_sync(0xffffffffu, in ? c : 0u);
-          if ((int)p == pp) {
-            bits = bal;
-            nsrc += sum;
-          }
-        }
-      } else {
-        nsrc += total;
-      }
-      // source b0 + lane of the stream (its cell's bit in t)
-      const uint32_t base = jb - excl;
-      uint32_t px = 0, py = 0, pz = 0, t = 0;
-      auto fetch = [&](uint32_t b0) {
-        const uint32_t g1 = min(b0 + (uint32_t)lane, total - 1);
-        const uint32_t before = __ballot_sync(0xffffffffu, valid && excl < b0);
-        const uint32_t rel = excl - b0;
-        const uint32_t heads = __reduce_or_sync(0xffffffffu, valid && rel < 32u ? 1u << rel : 0u);
-        t = __popc(before) + __popc(heads & (0xffffffffu >> (31u - (g1 - b0)))) - 1;
-        const uint32_t j = __shfl_sync(0xffffffffu, base, (int)t) + g1;
-        px = __ldg(A.x + j);
-        py = __ldg(A.y + j);
-        pz = __ldg(A.z + j);
+  float4 *win = reinterpret_cast<float4 *>(stage + 2 * kBatch);
+  for (uint32_t r0 = 0; r0 < k.C; r0 += 32u * (uint32_t)S) {
+    const uint32_t w0 = r0 + 32u * (uint32_t)s;
+    if (w0 < k.C) {
+      uint32_t excl, total, bits, t = 0;
+      __syncwarp();  // the previous window's table and last batch are read
+      k.window(A, w0, hc, lane, win, excl, total, bits, nsrc);
+      __syncwarp();
+      float4 nq = make_float4(0.f, 0.f, 0.f, 0.f);
+      auto fetch = [&](uint32_t b) {
+        const uint32_t g1 = min(b + (uint32_t)lane, total - 1);
+        t = stream_slot(excl, b, g1);
+        nq = __ldg(A.src + (__float_as_uint(win[t].w) + g1));
       };
-      uint32_t b0 = 32u * bs;
-      int flip = 0;
-      if (b0 < total) fetch(b0);
-      __syncwarp();  // the previous window's last batch is read
-      for (; b0 < total; b0 += 32u * bS) {
-        float *sb = stage + flip;
-        flip ^= kStage / 2;
-        const bool on = b0 + (uint32_t)lane < total;
-        sb[rec] = on ? (float)(int32_t)(ox - px) * sc : kFar;
-        sb[rec + 2] = (float)(int32_t)(oy - py) * sc;
-        sb[recz] = (float)(int32_t)(oz - pz) * sc;
-        if (SPARSE) sb[recz + 2] = __uint_as_float(on ? 1u << t : 0u);
+      float *sb = stage;
+      if (total) fetch(0u);
+      for (uint32_t b = 0; b < total; b += 32u) {
+        stage_source<true>(sb, win[t], nq, t, b + (uint32_t)lane < total, lane);
         __syncwarp();
-        const uint32_t n = total - b0;
-        if (b0 + 32u * bS < total) fetch(b0 + 32u * bS);
-        if (n >= 32) {
-#pragma unroll 8
-          for (int pr = 0; pr < 16; pr++)
-            pair_term<KERNEL, POT, SPARSE>(sb, pr, bits, X, Y, Z, H2, h2, hinv, hinv3, ax, ay, az,
-                                           ap);
-        } else {
-          const int np = (int)(n + 1) >> 1;
-#pragma unroll 2
-          for (int pr = 0; pr < np; pr++)
-            pair_term<KERNEL, POT, SPARSE>(sb, pr, bits, X, Y, Z, H2, h2, hinv, hinv3, ax, ay, az,
-                                           ap);
-        }
+        if (b + 32u < total) fetch(b + 32u);
+        eval_batch<KERNEL, POT, true, 1>(sb, total - b, bits, sink, soft);
+        sb = sb == stage ? stage + kBatch : stage;
       }
     }
-    if (!HEAVY) {
-      if (S == 1)
-        add(take());
-      else
-        share((int)min((uint32_t)S, (C - r0 + 31u) / 32u));
-    }
-  }
-  if (HEAVY) share(8);
-  if (A.inter && (!HEAVY || s == 0)) {
-    unsigned long long c;
-    if (SPARSE)
-      c = __reduce_add_sync(0xffffffffu, act ? nsrc : 0u);
-    else
-      c = (unsigned long long)nsrc * cd.y;
-    if (lane == 0 && c) atomicAdd(A.inter, c);
-  }
-  if (s > 0) return true;
-  // added to the far field (L2P, with GM) already in the force buffers, or
-  // stored into the near-field buffers when the two run side by side; the
-  // product is rounded on its own (no fused multiply-add into the far
-  // field), so that both forms add the same two values
-  if (act) {
-    const float GM = __ldg(A.box_gm + (key >> (3 * A.mbits)));
-    const float gx = __fmul_rn(GM, -nx), gy = __fmul_rn(GM, -ny), gz = __fmul_rn(GM, -nz);
-    if (A.store) {
-      A.ofx[i] = gx;
-      A.ofy[i] = gy;
-      A.ofz[i] = gz;
-      if (POT) A.opot[i] = __fmul_rn(GM, -np);
+    const float4 v = take<POT>(sink[0]);
+    if (S == 1) {
+      add(tot, v);
     } else {
-      A.ofx[i] += gx;
-      A.ofy[i] += gy;
-      A.ofz[i] += gz;
-      if (POT) A.opot[i] += __fmul_rn(GM, -np);
+      __syncwarp();  // every lane is done with this warp's staging
+      if (s > 0) reinterpret_cast<float4 *>(stage)[lane] = v;
+      group_sync(S, group);
+      if (s == 0) {
+        add(tot, v);
+        const int nw = (int)min((uint32_t)S, (k.C - r0 + 31u) / 32u);
+        for (int u = 1; u < nw; u++) add(tot, reinterpret_cast<const float4 *>(stage + u * kStage)[lane]);
+      }
+      group_sync(S, group);
     }
   }
+  if (A.inter) {
+    const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)lane < cd.y ? nsrc : 0u);
+    if (lane == 0 && c) atomicAdd(A.inter, (unsigned long long)c);
+  }
+  if (s == 0 && (uint32_t)lane < cd.y) write_sink<POT>(A, k.idx[0], k.key, tot);
   return true;
 }
 
-// The dense chunks and after them the sparse ones, taken from a device
-// counter by groups of S warps; blocks are persistent.  S = 1 wherever the chunks
-// alone fill the warps the GPU holds (A.warps); fewer chunks are shared by
-// 2, 4 or 8 warps each (12^3 particles on a 16^3 mesh are 64 chunks: 48 us
-// with one warp each on 7 blocks).  HEAVY: the second launch, eight warps on
-// each chunk that the first one listed.  The sums depend neither on S nor on the
-// launch shape, and the heavy rule only on a chunk's neighbourhood.
-template <int KERNEL, bool POT, bool HEAVY>
-__global__ void __launch_bounds__(256, 4) near_stream_kernel(const NearArgs A) {
+// The sparse chunks, taken from a device counter by groups of S warps; blocks
+// are persistent.  S = 1 wherever the chunks alone fill the warps the GPU
+// holds (A.warps); fewer are shared by 2, 4 or 8 warps each (12^3 particles on
+// a 16^3 mesh are 64 chunks: 48 us with one warp each on 7 blocks).  The sums
+// do not depend on S.
+template <int KERNEL, bool POT>
+__global__ void __launch_bounds__(256, 4) near_sparse_kernel(const NearArgs A) {
   __shared__ __align__(16) float stage[8 * kStage];
   __shared__ uint32_t taken_s[2][8];  // by the parity of the turn: one barrier a turn
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const uint32_t nd = *A.ndense, ns = A.nsparse ? *A.nsparse : 0u;
-  const uint2 *sch = A.soff ? A.schunks + *A.soff : A.schunks;
-  const uint32_t nch = HEAVY ? A.work[1] : nd + ns;
+  const uint32_t nch = *A.nsparse;
+  const uint2 *list = A.soff ? A.schunks + *A.soff : A.schunks;
   int S = 8;
-  if (!HEAVY)
-    while (S > 1 && (size_t)nch * S > A.warps) S >>= 1;
+  while (S > 1 && (size_t)nch * S > A.warps) S >>= 1;
   const int s = wib & (S - 1), group = wib / S;
   // maxch > 0: a group takes at most maxch chunks and the block then exits,
   // so that blocks of kernels on other streams get the SM in between
-  for (uint32_t taken = 0; HEAVY || A.maxch == 0 || taken < A.maxch; taken++) {
+  for (uint32_t taken = 0; A.maxch == 0 || taken < A.maxch; taken++) {
     uint32_t ch = 0;
     if (S > 1) {
-      if (s == 0 && lane == 0) taken_s[taken & 1][group] = atomicAdd(A.work + (HEAVY ? 2 : 0), 1u);
+      if (s == 0 && lane == 0) taken_s[taken & 1][group] = atomicAdd(A.work, 1u);
       group_sync(S, group);
       ch = taken_s[taken & 1][group];
     } else {
@@ -505,18 +575,142 @@ __global__ void __launch_bounds__(256, 4) near_stream_kernel(const NearArgs A) {
       ch = __shfl_sync(0xffffffffu, ch, 0);
     }
     if (ch >= nch) break;
-    if (HEAVY) ch = A.heavy[ch];
-    float *st = stage + wib * kStage;
-    const bool done =
-        ch < nd
-            ? near_chunk<KERNEL, POT, false, HEAVY>(A, A.dchunks[ch], s, S, group, st, lane)
-            : near_chunk<KERNEL, POT, true, HEAVY>(A, sch[ch - nd], s, S, group, st, lane);
-    if (!done && s == 0 && lane == 0) A.heavy[atomicAdd(A.work + 1, 1u)] = ch;
+    if (!sparse_chunk<KERNEL, POT>(A, list[ch], s, S, group, stage + wib * kStage, lane) &&
+        s == 0 && lane == 0)
+      A.heavy[atomicAdd(A.work + 1, 1u)] = ch;
   }
 }
 
-// Sparse chunks cell by cell (tuning sparse_path 1, and meshes of 8, where a
-// block-sized frame is not smaller than half the box): one warp per chunk; each
+// Dense chunks and heavy sparse ones: a block each.  The eight warps tabulate
+// eight windows at a time, one each, and take the segments of kSeg sources of these
+// windows in turn; their sums are added in warp order at the end.  A chunk
+// then takes a few us, so that the last ones leave no tail (a warp each: 64^3
+// particles in Plummer spheres had 2200 dense chunks for 3552 warps, and the
+// launch half idle).  NS sinks per lane: a dense chunk of more than 32 sinks
+// holds two, so that each staged quad feeds eight interactions.
+constexpr uint32_t kSeg = 256;
+struct CoopSmem {
+  float stage[8][2 * kBatch];
+  float4 win[8][32];
+  uint32_t excl[8][32], bits[8][32], total[8];
+  uint32_t chunk[2];
+};
+
+template <int KERNEL, bool POT, bool SPARSE, int NS>
+__device__ __forceinline__ void coop_chunk(const NearArgs &A, const uint2 cd, CoopSmem &sm,
+                                           int wib, int lane) {
+  Chunk<SPARSE, NS> k;
+  k.open(A, cd, lane);
+  const float hc = 1.0f / (float)(1 << A.mbits);
+  Sink sink[NS];
+  k.sinks(A, hc, sink);
+  const Soft soft(A.soft);
+  uint32_t nsrc = 0;
+  for (uint32_t r0 = 0; r0 < k.C; r0 += 256u) {
+    const uint32_t w0 = r0 + 32u * (uint32_t)wib;
+    uint32_t excl = 0xffffffffu, total = 0, bits = 0;
+    if (r0) __syncthreads();  // the previous round's tables are read
+    if (w0 < k.C) k.window(A, w0, hc, lane, sm.win[wib], excl, total, bits, nsrc);
+    sm.excl[wib][lane] = excl;
+    if (SPARSE) sm.bits[wib][lane] = bits;
+    if (lane == 0) sm.total[wib] = total;
+    __syncthreads();
+    // this warp's place: window w, batch at b of its tot sources; segments
+    // are numbered through the windows, this warp's are wib, wib + 8, ...
+    uint32_t w = 0, b = 0, tot = sm.total[0], skip = (uint32_t)wib;
+    auto seek = [&]() {  // to the segment `skip` segments on from (w, b); w = 8: none
+      for (;;) {
+        const uint32_t left = b < tot ? (tot - b + kSeg - 1) / kSeg : 0u;
+        if (skip < left) {
+          b += skip * kSeg;
+          break;
+        }
+        skip -= left;
+        b = 0;
+        if (++w == 8) break;
+        tot = sm.total[w];
+      }
+      if (w < 8) {
+        excl = sm.excl[w][lane];
+        if (SPARSE) bits = sm.bits[w][lane];
+      }
+    };
+    seek();
+    uint32_t t = 0;
+    float4 nq = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto fetch = [&]() {
+      const uint32_t g1 = min(b + (uint32_t)lane, tot - 1);
+      t = stream_slot(excl, b, g1);
+      nq = __ldg(A.src + (__float_as_uint(sm.win[w][t].w) + g1));
+    };
+    float *sb = sm.stage[wib];
+    if (w < 8) fetch();
+    __syncwarp();  // the last batch of the round before is read
+    while (w < 8) {
+      stage_source<SPARSE>(sb, sm.win[w][t], nq, t, b + (uint32_t)lane < tot, lane);
+      __syncwarp();
+      const uint32_t n = tot - b, eb = bits;
+      b += 32u;
+      if (b % kSeg == 0u || b >= tot) {  // the segment's end: seven segments on
+        skip = 7u;
+        if (b >= tot) b = tot;
+        seek();
+      }
+      if (w < 8) fetch();
+      eval_batch<KERNEL, POT, SPARSE, NS>(sb, n, eb, sink, soft);
+      sb = sb == sm.stage[wib] ? sm.stage[wib] + kBatch : sm.stage[wib];
+    }
+  }
+  // the eight warps' sums, in order
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < NS; u++)
+    reinterpret_cast<float4 *>(sm.stage[wib])[32 * u + lane] = take<POT>(sink[u]);
+  if (A.inter) {  // (each warp has counted its own windows)
+    unsigned long long c;
+    if (SPARSE)
+      c = __reduce_add_sync(0xffffffffu, (uint32_t)lane < cd.y ? nsrc : 0u);
+    else
+      c = (unsigned long long)nsrc * cd.y;
+    if (lane == 0 && c) atomicAdd(A.inter, c);
+  }
+  __syncthreads();
+  if (wib < NS) {  // warp u: the lanes' sinks u
+    float4 n = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int v = 0; v < 8; v++) add(n, reinterpret_cast<const float4 *>(sm.stage[v])[32 * wib + lane]);
+    const uint32_t e = (uint32_t)(lane + 32 * wib);
+    if (e < cd.y) write_sink<POT>(A, SPARSE ? k.idx[0] : cd.x + e, k.key, n);
+  }
+}
+
+template <int KERNEL, bool POT>
+__global__ void __launch_bounds__(256, 3) near_coop_kernel(const NearArgs A) {
+  __shared__ __align__(16) CoopSmem sm;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const uint32_t nh = A.nsparse ? A.work[1] : 0u, nch = nh + *A.ndense;
+  const uint2 *sch = A.soff ? A.schunks + *A.soff : A.schunks;
+  if (threadIdx.x == 0) sm.chunk[0] = atomicAdd(A.work + 2, 1u);
+  for (uint32_t taken = 0; A.maxch == 0 || taken < 8 * A.maxch; taken++) {
+    __syncthreads();  // the chunk's number is there, the previous chunk's sums are read
+    const uint32_t ch = sm.chunk[taken & 1];
+    if (ch >= nch) break;
+    // the next one, asked for early (none that this block would not take)
+    if (threadIdx.x == 0 && (A.maxch == 0 || taken + 1 < 8 * A.maxch))
+      sm.chunk[(taken + 1) & 1] = atomicAdd(A.work + 2, 1u);
+    if (ch < nh) {
+      coop_chunk<KERNEL, POT, true, 1>(A, sch[A.heavy[ch]], sm, wib, lane);
+    } else {
+      const uint2 cd = A.dchunks[ch - nh];
+      if (cd.y <= 32)
+        coop_chunk<KERNEL, POT, false, 1>(A, cd, sm, wib, lane);
+      else
+        coop_chunk<KERNEL, POT, false, 2>(A, cd, sm, wib, lane);
+    }
+  }
+}
+
+// Sparse chunks cell by cell (tuning sparse_path 1): one warp per chunk; each
 // candidate cell's sources are staged as their own batch, and a lane takes part only
 // where the cell lies in its own stencil window (lo2 < |o|^2 <= hi2).
 template <int KERNEL, bool POT>
@@ -780,9 +974,6 @@ NearArgs near_args(ct2g_ctx *ctx, const unsigned long long *stm, float lo2, floa
   A.walk = make_walk(ctx->mbits);
   A.skeys = ctx->keys;
   A.rbegin = (uint32_t)ctx->rung_begin;
-  A.x = ctx->x;
-  A.y = ctx->y;
-  A.z = ctx->z;
   A.src = ctx->src;
   A.mbits = ctx->mbits;
   A.soft = ctx->opt.hsoft;
@@ -796,6 +987,7 @@ NearArgs near_args(ct2g_ctx *ctx, const unsigned long long *stm, float lo2, floa
   A.opot = pot;
   A.store = store;
   A.heavy = ctx->keys2;  // binning scratch: as many entries as particles, free by now
+  A.heavy_min = heavy_min(ctx->M);
   A.warps = (uint32_t)ctx->num_sms * 32u;
   return A;
 }
@@ -818,21 +1010,20 @@ unsigned near_grid(const ct2g_ctx *ctx, int per_sm, const NearArgs &A) {
   return (unsigned)std::max<size_t>(1, blocks);
 }
 
-// dense and sparse chunks of A, then the heavy ones among them
+// the sparse chunks of A, then the dense and the heavy ones
 template <int K, bool POT>
 int launch_stream(ct2g_ctx *ctx, const NearArgs &A, cudaStream_t st) {
   int per_sm = 0;
-  auto k = near_stream_kernel<K, POT, false>;
+  if (A.nsparse) {
+    auto k = near_sparse_kernel<K, POT>;
+    CT2G_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 256, 0));
+    k<<<near_grid(ctx, per_sm, A), 256, 0, st>>>(A);
+    CT2G_LAUNCHED(ctx);
+  }
+  auto k = near_coop_kernel<K, POT>;
   CT2G_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 256, 0));
   k<<<near_grid(ctx, per_sm, A), 256, 0, st>>>(A);
   CT2G_LAUNCHED(ctx);
-  auto kh = near_stream_kernel<K, POT, true>;
-  CT2G_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kh, 256, 0));
-  const size_t nr = ctx->n - ctx->rung_begin;
-  if (nr > kHeavySources) {  // fewer particles than a heavy chunk has sources: none
-    kh<<<near_grid(ctx, per_sm, A), 256, 0, st>>>(A);
-    CT2G_LAUNCHED(ctx);
-  }
   return CT2G_OK;
 }
 
@@ -845,10 +1036,6 @@ int launch_cells(ct2g_ctx *ctx, const NearArgs &A, cudaStream_t st) {
   CT2G_LAUNCHED(ctx);
   return CT2G_OK;
 }
-
-// the streamed sparse form works in a frame of up to 8 cells from its origin,
-// which has to be less than half the box
-bool stream_sparse(const ct2g_ctx *ctx) { return ctx->sparse_path == 2 && ctx->M >= 16; }
 
 // the dense chunks (counts[0]) and the sparse sinks: streamed with them as the
 // per-block chunks stored after the dense ones (counts[2]; sparse_path 2), the
@@ -868,7 +1055,7 @@ int launch_near(ct2g_ctx *ctx, cudaStream_t st, float *fx, float *fy, float *fz,
   // mesh kernels' blocks in
   A.maxch = store ? (uint32_t)ctx->near_chunks_per_warp : 0u;
   A.inter = ctx->d_inter;
-  const bool stream = stream_sparse(ctx);
+  const bool stream = ctx->sparse_path == 2;
   if (stream) A.nsparse = c + 2;
   CT2G_TRY((launch_stream<K, POT>(ctx, A, st)));
   if (stream) return CT2G_OK;
@@ -918,7 +1105,7 @@ int ct2g_near_window(ct2g_ctx *ctx, const uint2 *dch, const uint32_t *nd, const 
   A.schunks = sch;
   A.slist = slist;
   A.work = work;
-  const bool stream = stream_sparse(ctx), plummer = ctx->opt.kernel != CT2G_SOFT_SPHERE;
+  const bool stream = ctx->sparse_path == 2, plummer = ctx->opt.kernel != CT2G_SOFT_SPHERE;
   if (stream) A.nsparse = ns;
   if (plummer)
     CT2G_TRY((pot ? launch_stream<CT2G_SOFT_PLUMMER, true>(ctx, A, ctx->stream)

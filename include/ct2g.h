@@ -241,8 +241,8 @@ int ct2g_batch_destroy(ct2g_batch *b);
  * the union of their stencils go in windows of 32, every lane holds a bit
  * mask of those that lie in its own stencil, and the window's sources are
  * streamed in full batches of 32 staged in shared memory, each evaluated by
- * every lane (meshes of 8 take 1); 1: the same chunks, the union walked cell
- * by cell, each cell's sources staged as their own batch; 0: one sparse sink per warp lane, each
+ * every lane; 1: the same chunks, the union walked cell by cell, each cell's
+ * sources staged as their own batch; 0: one sparse sink per warp lane, each
  * lane walking its own stencil and reading its own sources (no masked work,
  * but every lane gathers its own sources through the L1 cache); overlap -- 1: the near field runs on a second stream
  * beside the mesh solve (from the end of binning to the L2P pass) into its

@@ -17,6 +17,7 @@ pytestmark = pytest.mark.gpu
     (1, 4, 2.0, 0, 1, 0.02),
     (33, 3, 3.0, 1, 1, 0.05),
     (700, 3, 2.5, 0, 2, 0.05),
+    (6000, 3, 3.0, 0, 1, 0.03),
     (1728, 4, 4.0, 1, 3, 0.03),
     (20011, 5, 4.0, 0, 40, 0.02),
     (20011, 5, 3.0, 1, 1, 0.02),
