@@ -1,0 +1,4 @@
+// mesh-solve kernels of order 6
+#include "ct2g_fft_mesh.cuh"
+
+CT2G_FFT_ORDER_FNS(6)

@@ -433,6 +433,15 @@ int ct2g_mesh_solve(ct2g_ctx *ctx, bool fused_l2p, bool pot, int p2m = CT2G_P2M_
 int ct2g_spec_forward(ct2g_ctx *ctx, int src);
 int ct2g_spec_mg2l(ct2g_ctx *ctx);
 int ct2g_spec_inverse(ct2g_ctx *ctx, bool l2p, bool pot);
+// one order's mesh-solve kernels (ct2g_fft_p1.cu ... p6.cu): its constants,
+// stage 0 / 1 / 2 (z pass, fused X pass + MG2L, inverse z pass), the plane
+// pipeline (*done: it ran), and whether the fused X pass fits a mesh
+struct Ct2gOrderFns {
+  int (*consts)(ct2g_ctx *ctx);
+  int (*stage)(ct2g_ctx *ctx, int stage, int mode);
+  int (*pipe)(ct2g_ctx *ctx, bool inverse, int mode, bool *done);
+  bool (*fx_fits)(int N);
+};
 // the X passes and MG2L run as one kernel for this context
 bool ct2g_mg2l_fused(const ct2g_ctx *ctx);
 // MG2L alone on ctx->spec (ct2g_mesh.cu)
