@@ -75,7 +75,7 @@ void free_particles(ct2g_ctx *ctx) {
   void *ptrs[] = {ctx->x, ctx->y, ctx->z, ctx->id, ctx->vx, ctx->vy, ctx->vz, ctx->rung,
                   ctx->x2, ctx->y2, ctx->z2, ctx->id2, ctx->vx2, ctx->vy2, ctx->vz2, ctx->rung2,
                   ctx->keys, ctx->keys2, ctx->vals, ctx->vals2, ctx->hist, ctx->src,
-                  ctx->chunks, ctx->sparse_list, ctx->flags, ctx->fx,
+                  ctx->chunks, ctx->schunks, ctx->sparse_list, ctx->flags, ctx->fx,
                   ctx->fy, ctx->fz,
                   ctx->pot, ctx->nfx, ctx->nfy, ctx->nfz, ctx->npot, ctx->cmom, ctx->p2m_big};
   for (void *p : ptrs)
@@ -88,7 +88,7 @@ void free_particles(ct2g_ctx *ctx) {
   ctx->rung2 = nullptr;
   ctx->keys = ctx->keys2 = ctx->vals = ctx->vals2 = ctx->hist = nullptr;
   ctx->src = nullptr;
-  ctx->chunks = nullptr;
+  ctx->chunks = ctx->schunks = nullptr;
   ctx->sparse_list = ctx->flags = nullptr;
   ctx->fx = ctx->fy = ctx->fz = ctx->pot = nullptr;
   ctx->nfx = ctx->nfy = ctx->nfz = ctx->npot = nullptr;
@@ -205,7 +205,8 @@ int ct2g_alloc_particles(ct2g_ctx *ctx, size_t n) {
   free_particles(ctx);
   ctx->epoch++;
   const size_t cap = n;
-  const size_t ntiles = (cap + 4095) / 4096;
+  // radix tiles: 4096 items, 1024 up to 65536 particles (64 tiles at most)
+  const size_t ntiles = std::max<size_t>((cap + 4095) / 4096, std::min<size_t>((cap + 1023) / 1024, 64));
 #define A(ptr, bytes) CT2G_CUDA(ctx, cudaMalloc(&(ptr), (bytes)))
   A(ctx->x, cap * 4);
   A(ctx->y, cap * 4);
@@ -227,9 +228,10 @@ int ct2g_alloc_particles(ct2g_ctx *ctx, size_t n) {
   A(ctx->keys2, cap * 4);
   A(ctx->vals, cap * 4);
   A(ctx->vals2, cap * 4);
-  A(ctx->hist, ntiles * 256 * 4);
+  A(ctx->hist, ntiles * 512 * 4);
   A(ctx->src, cap * sizeof(float4));
   A(ctx->chunks, cap * sizeof(uint2));
+  A(ctx->schunks, cap * sizeof(uint2));
   A(ctx->sparse_list, cap * 4);
   A(ctx->flags, cap * 4);
   A(ctx->fx, cap * 4);
@@ -243,10 +245,10 @@ int ct2g_alloc_particles(ct2g_ctx *ctx, size_t n) {
 #undef A
   ctx->cap = cap;
   if (ctx->p2m_compact) CT2G_TRY(ct2g_alloc_p2m_compact(ctx));
-  // scan scratch for the largest scan of a step (radix histograms, cell
-  // ranges, per-particle flags), so that no step allocates
+  // scan scratch for the largest scan of a step (radix histograms, block
+  // ranks, per-particle flags), so that no step allocates
   const size_t words = ct2g_scan_scratch_words(
-      std::max<size_t>(std::max<size_t>(ntiles * 256, (size_t)ctx->CB + 1), cap));
+      std::max<size_t>(std::max<size_t>(ntiles * 512, (size_t)ctx->CB / 64), cap));
   if (ctx->scan_tmp_words < words) {
     if (ctx->scan_tmp) cudaFree(ctx->scan_tmp);
     ctx->scan_tmp = nullptr;

@@ -252,8 +252,7 @@ struct ct2g_ctx {
   unsigned long long *occ = nullptr;  // [C/64] occupancy bits of 4x4x4 cell blocks
   unsigned long long *stmask = nullptr;  // [64][27] stencil bits per (in-block cell, block offset)
   float4 *src = nullptr;           // per sorted particle: offset from own cell centre
-  uint2 *chunks = nullptr;         // near-field warp chunks (start, count): dense ones
-                                   // (particle index) then sparse ones (sparse_list index)
+  uint2 *chunks = nullptr;         // near-field dense chunks (particle index, sinks)
   uint32_t *sparse_list = nullptr; // particles of sparse cells, in order
   uint32_t *flags = nullptr;
   // work-list sizes stay on the device, so a step needs no host readback:
@@ -336,6 +335,7 @@ struct ct2g_ctx {
   bool forces_valid = false;
   bool pot_valid = false;        // potential computed with the current forces
   bool has_particles = false;
+  uint2 *schunks = nullptr;      // near-field sparse chunks (sparse_list index, sinks)
 };
 
 // ---------------------------------------------------------------------------

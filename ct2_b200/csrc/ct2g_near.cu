@@ -136,8 +136,7 @@ struct NearArgs {
   const uint2 *dchunks;     // dense chunks (first particle, sinks), *ndense of them
   const uint32_t *ndense;
   const uint2 *schunks;     // sparse chunks (first sparse_list entry, sinks),
-  const uint32_t *soff;     // starting at schunks[*soff] (null: 0), *nsparse of
-  const uint32_t *nsparse;  // them (null: none)
+  const uint32_t *nsparse;  // *nsparse of them (null: none)
   const uint32_t *slist;
   const uint32_t *cs;
   const unsigned long long *occ, *stm;
@@ -558,7 +557,7 @@ __global__ void __launch_bounds__(256, 4) near_sparse_kernel(const NearArgs A) {
   __shared__ uint32_t taken_s[2][8];  // by the parity of the turn: one barrier a turn
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t nch = *A.nsparse;
-  const uint2 *list = A.soff ? A.schunks + *A.soff : A.schunks;
+  const uint2 *list = A.schunks;
   int S = 8;
   while (S > 1 && (size_t)nch * S > A.warps) S >>= 1;
   const int s = wib & (S - 1), group = wib / S;
@@ -689,7 +688,6 @@ __global__ void __launch_bounds__(256, 3) near_coop_kernel(const NearArgs A) {
   __shared__ __align__(16) CoopSmem sm;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t nh = A.nsparse ? A.work[1] : 0u, nch = nh + *A.ndense;
-  const uint2 *sch = A.soff ? A.schunks + *A.soff : A.schunks;
   if (threadIdx.x == 0) sm.chunk[0] = atomicAdd(A.work + 2, 1u);
   for (uint32_t taken = 0; A.maxch == 0 || taken < 8 * A.maxch; taken++) {
     __syncthreads();  // the chunk's number is there, the previous chunk's sums are read
@@ -699,7 +697,7 @@ __global__ void __launch_bounds__(256, 3) near_coop_kernel(const NearArgs A) {
     if (threadIdx.x == 0 && (A.maxch == 0 || taken + 1 < 8 * A.maxch))
       sm.chunk[(taken + 1) & 1] = atomicAdd(A.work + 2, 1u);
     if (ch < nh) {
-      coop_chunk<KERNEL, POT, true, 1>(A, sch[A.heavy[ch]], sm, wib, lane);
+      coop_chunk<KERNEL, POT, true, 1>(A, A.schunks[A.heavy[ch]], sm, wib, lane);
     } else {
       const uint2 cd = A.dchunks[ch - nh];
       if (cd.y <= 32)
@@ -803,7 +801,7 @@ __global__ void __launch_bounds__(256, 4) near_cells_kernel(const NearArgs A) {
   __shared__ float4 sbuf[8][32];  // one batch of 32 sources per warp
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t nch = *A.nsparse;
-  const uint2 *list = A.soff ? A.schunks + *A.soff : A.schunks;
+  const uint2 *list = A.schunks;
   for (uint32_t taken = 0; A.maxch == 0 || taken < A.maxch; taken++) {
     uint32_t ch = 0;
     if (lane == 0) ch = atomicAdd(A.work, 1u);
@@ -1038,7 +1036,7 @@ int launch_cells(ct2g_ctx *ctx, const NearArgs &A, cudaStream_t st) {
 }
 
 // the dense chunks (counts[0]) and the sparse sinks: streamed with them as the
-// per-block chunks stored after the dense ones (counts[2]; sparse_path 2), the
+// per-block chunks (counts[2]; sparse_path 2), the
 // same chunks cell by cell (sparse_path 1), or one sink per lane (sparse_path
 // 0, counts[1] of them); work counters counts[8..11]
 template <int K, bool POT>
@@ -1047,8 +1045,9 @@ int launch_near(ct2g_ctx *ctx, cudaStream_t st, float *fx, float *fy, float *fz,
   uint32_t *c = ctx->d_counts;
   NearArgs A = near_args(ctx, ctx->stmask, -1.f, ctx->opt.bwidth * ctx->opt.bwidth, fx, fy, fz, pot,
                          store);
-  A.dchunks = A.schunks = ctx->chunks;
-  A.ndense = A.soff = c;
+  A.dchunks = ctx->chunks;
+  A.schunks = ctx->schunks;
+  A.ndense = c;
   A.slist = ctx->sparse_list;
   A.work = c + 8;
   // capped warps only beside the mesh solve (overlap), where they let the
