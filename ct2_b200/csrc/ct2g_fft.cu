@@ -30,8 +30,10 @@ namespace {
 // LP complex (packed) lines per block; npairs = number of real-line pairs;
 // output rows hold ld >= N/2+1 complex (the rest is written as zero).  VEC:
 // ld*sizeof(complex) is a multiple of 16 bytes.
+// (FP32 up to N = 256: four blocks per SM, whose loads and stores then overlap
+// the others' transforms; larger in-register DFTs and FP64 need the registers)
 template <typename T, int N, bool VEC>
-__global__ void __launch_bounds__(256, 3) fftz_r2c_kernel(const T *__restrict__ in,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 && N <= 256 ? 4 : 3) fftz_r2c_kernel(const T *__restrict__ in,
                                                           typename Cplx<T>::type *__restrict__ out,
                                                           size_t npairs, int LP, int ld,
                                                           const typename Cplx<T>::type *__restrict__ tw) {
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(256, 3) fftz_r2c_kernel(const T *__restrict__ 
 
 // ---- pass Z inverse: pairs of half spectra -> real lines --------------------
 template <typename T, int N, bool VEC>
-__global__ void __launch_bounds__(256, 3) fftz_c2r_kernel(const typename Cplx<T>::type *__restrict__ in,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 && N <= 256 ? 4 : 3) fftz_c2r_kernel(const typename Cplx<T>::type *__restrict__ in,
                                                           T *__restrict__ out, size_t npairs, int LP,
                                                           int ld,
                                                           const typename Cplx<T>::type *__restrict__ tw) {
@@ -176,7 +178,9 @@ __global__ void __launch_bounds__(256, 3) fft_cols_kernel(C2 *__restrict__ a, si
     if (c < wv) *reinterpret_cast<V *>(s + r * W + c) = *reinterpret_cast<const V *>(base + (size_t)r * rstride + c);
   }
   __syncthreads();
-  tile_fft<N, false, C2, INV>(s, W, W, stw);
+  // (the last tile of a half spectrum holds one column: its own, not W)
+  if (wv == W) tile_fft<N, false, C2, INV>(s, W, W, stw);
+  else tile_fft<N, false, C2, INV>(s, wv, W, stw);
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * CH; e += 256) {
     const int r = e / CH, c = (e % CH) * CPC;
@@ -426,7 +430,6 @@ int run_cols(ct2g_ctx *ctx, typename Cplx<T>::type *spec, int batch, bool inv, s
              bool full = false) {
   using C2 = typename Cplx<T>::type;
   const size_t NH = full ? (size_t)N : (size_t)N / 2 + 1;
-  const bool vec = (ld * sizeof(C2)) % 16 == 0;
   for (int pass = 0; pass < 2; pass++) {
     const bool ypass = (pass == 0) != inv;
     size_t nouter, ostride, rstride, ncols;
@@ -441,6 +444,12 @@ int run_cols(ct2g_ctx *ctx, typename Cplx<T>::type *spec, int batch, bool inv, s
       rstride = (size_t)N * ld;
       ncols = (size_t)N * ld;
     }
+    // rows on 16-byte boundaries: the x pass's always are (N rows of ld values
+    // apart), the y pass's where ld is even (FP32), if the grid itself is.  (The x
+    // passes of 3 x 256^3 half spectra moved their tiles by plain 8-byte loads like the
+    // y passes, 117 us each; by TMA 74 us.  Feeding the y passes by 8-byte cp.async
+    // or in tiles of 32 columns measured 136 and 119 us.)
+    const bool vec = (rstride * sizeof(C2)) % 16 == 0 && ((uintptr_t)spec & 15) == 0;
     if constexpr (sizeof(C2) == 8 && (N == 256 || N == 512)) {
       if (ctx->fft_tc) {
         CT2G_TRY(ct2g_fft_cols_tc(ctx, spec, N, nouter, ostride, rstride, ncols, inv));
