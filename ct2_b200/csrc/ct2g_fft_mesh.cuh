@@ -3,6 +3,9 @@
 // file of its own (ct2g_fft_p1.cu ... p6.cu).
 #pragma once
 
+#include <type_traits>
+#include <utility>
+
 #include "ct2g_fft_core.cuh"
 
 namespace {
@@ -61,70 +64,76 @@ __device__ __forceinline__ void p2m_accumulate(const uint32_t *__restrict__ px,
   for (int k = K0; k < K1; k++) acc[k - K0] += qx[T.nx[k]] * qy[T.ny[k]] * qz[T.nz[k]];
 }
 
+// v[k] summed over the warp, k < K <= 32: each lane ends with the sum of the one k
+// it returns (-1: none) in v[0].  At each step a lane hands half of its values to
+// its partner and adds what it is handed to the others, so K values take about
+// K + 4 exchanges instead of 5 K (each two shuffles, the pipe that held a warp's
+// cell); each sum is the same tree as a butterfly per value.
+template <int K>
+__device__ __forceinline__ int warp_sums(double (&v)[K], int lane) {
+  static_assert(K <= 32, "a value per lane at most");
+  int base = 0, cnt = K;
+#pragma unroll
+  for (int s = 0; s < 5; s++) {
+    const int n = (K + (1 << s) - 1) >> s, h = (n + 1) >> 1, o = 16 >> s;
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < (K + 1) / 2; k++) {
+      if (k < h) {
+        const double lo = v[k], hi = k + h < n ? v[k + h < K ? k + h : 0] : 0.0;
+        v[k] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
+      }
+    }
+    base += up ? h : 0;
+    cnt = up ? max(cnt - h, 0) : min(cnt, h);
+  }
+  return cnt > 0 ? base : -1;
+}
+
 // the moments of cell particles b, b + step, ... < e (a thread: step 1; a
-// warp: lane offset, step 32, then summed over the warp) into the packed smem
-// lines at z, for components [K0, K1): the components go in two halves so
-// that only half of the FP64 sums are live at once
+// warp: lane offset, step 32 or more, then summed over the warp) for components
+// [K0, K1): the components go in pieces so that only one's FP64 sums are live at
+// once.  st(k, sum) by the lane that has it.
 template <int P, int K0, int K1, typename ST>
 __device__ __forceinline__ void p2m_sum(const uint32_t *__restrict__ px,
                                         const uint32_t *__restrict__ py,
                                         const uint32_t *__restrict__ pz, uint32_t b, uint32_t e,
-                                        uint32_t step, bool warp_sum, uint32_t ux, uint32_t uy,
-                                        uint32_t uz, bool write, ST st) {
+                                        uint32_t step, bool warp_sum, int lane, uint32_t ux,
+                                        uint32_t uy, uint32_t uz, ST st) {
   double acc[K1 - K0];
 #pragma unroll
   for (int k = 0; k < K1 - K0; k++) acc[k] = 0.0;
   for (uint32_t i = b; i < e; i += step) p2m_accumulate<P, K0, K1>(px, py, pz, i, ux, uy, uz, acc);
   if (warp_sum) {
-#pragma unroll
-    for (int k = 0; k < K1 - K0; k++) {
-      double v = acc[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      acc[k] = v;
-    }
-  }
-  if (write) {
+    const int k = warp_sums<K1 - K0>(acc, lane);
+    if (k >= 0) st(K0 + k, acc[0]);
+  } else {
 #pragma unroll
     for (int k = K0; k < K1; k++) st(k, acc[k - K0]);
   }
 }
-template <int P, int K0, int K1, typename ST>
-__device__ __forceinline__ void p2m_group(const uint32_t *__restrict__ px,
-                                          const uint32_t *__restrict__ py,
-                                          const uint32_t *__restrict__ pz, uint32_t b, uint32_t e,
-                                          uint32_t step, bool warp_sum, uint32_t ux, uint32_t uy,
-                                          uint32_t uz, bool write, ST st) {
-  p2m_sum<P, K0, K1>(px, py, pz, b, e, step, warp_sum, ux, uy, uz, write,
-                     [&](int k, double v) { st(k, (float)v); });
+
+// f(0), f(1), ... of NP pieces, as compile-time constants
+template <typename F, int... I>
+__device__ __forceinline__ void each_piece(F f, std::integer_sequence<int, I...>) {
+  (f(std::integral_constant<int, I>{}), ...);
 }
 
-// the same sums into the packed smem lines at z
-template <int P, int N, int K0, int K1>
-__device__ __forceinline__ void p2m_half(const uint32_t *__restrict__ px,
-                                         const uint32_t *__restrict__ py,
-                                         const uint32_t *__restrict__ pz, uint32_t b, uint32_t e,
-                                         uint32_t step, bool warp_sum, uint32_t ux, uint32_t uy,
-                                         uint32_t uz, int z, float *sr, bool write) {
-  using LL = LineLayout<N, true>;
-  p2m_group<P, K0, K1>(px, py, pz, b, e, step, warp_sum, ux, uy, uz, write,
-                       [&](int k, float v) { sr[2 * LL::at(k >> 1, z, 0) + (k & 1)] = v; });
-}
-
-// the warp-sized parts of a cell of more than kBlockCell particles: part v of
-// eight takes the particles 32 v + lane, + 256, ...; its sum over the warp
-// goes through st (lane 0)
-template <int P, typename ST>
-__device__ __forceinline__ void p2m_part(const uint32_t *__restrict__ px,
-                                         const uint32_t *__restrict__ py,
-                                         const uint32_t *__restrict__ pz, uint32_t b, uint32_t e,
-                                         int v, int lane, uint32_t ux, uint32_t uy, uint32_t uz,
-                                         ST st) {
+// all the components in NP pieces; st(piece, k, sum)
+template <int P, int NP, typename ST>
+__device__ __forceinline__ void p2m_all(const uint32_t *__restrict__ px,
+                                        const uint32_t *__restrict__ py,
+                                        const uint32_t *__restrict__ pz, uint32_t b, uint32_t e,
+                                        uint32_t step, bool warp_sum, int lane, uint32_t ux,
+                                        uint32_t uy, uint32_t uz, ST st) {
   constexpr int NC = ct2g_ncomp(P);
-  const uint32_t b0 = b + 32u * (uint32_t)v + (uint32_t)lane;
-  p2m_sum<P, 0, NC / 3>(px, py, pz, b0, e, 256, true, ux, uy, uz, lane == 0, st);
-  p2m_sum<P, NC / 3, 2 * NC / 3>(px, py, pz, b0, e, 256, true, ux, uy, uz, lane == 0, st);
-  p2m_sum<P, 2 * NC / 3, NC>(px, py, pz, b0, e, 256, true, ux, uy, uz, lane == 0, st);
+  each_piece(
+      [&](auto i) {
+        constexpr int I = decltype(i)::value;
+        p2m_sum<P, I * NC / NP, (I + 1) * NC / NP>(px, py, pz, b, e, step, warp_sum, lane, ux, uy,
+                                                   uz, [&](int k, double v) { st(I, k, v); });
+      },
+      std::make_integer_sequence<int, NP>{});
 }
 
 // ---- P2M into compact per-cell records ---------------------------------------
@@ -165,25 +174,20 @@ __device__ __forceinline__ void demorton(uint32_t key, int mbits, uint32_t &x, u
 }
 
 // the moments of the cell `key` (particles b .. e) into out (a thread: step
-// 1; a warp: lanes strided, summed over the warp, lane 0 writes)
+// 1; a warp: lanes strided, summed over the warp)
 template <int P>
 __device__ __forceinline__ void p2m_cell(const uint32_t *__restrict__ px,
                                          const uint32_t *__restrict__ py,
                                          const uint32_t *__restrict__ pz, uint32_t key, int mbits,
                                          uint32_t b, uint32_t e, bool warp, int lane,
                                          float *out) {
-  constexpr int NC = ct2g_ncomp(P);
   uint32_t cx, cy, cz;
   demorton(key, mbits, cx, cy, cz);
   const int sh = 32 - mbits;
   const uint32_t halfc = 1u << (sh - 1);
   const uint32_t ux = (cx << sh) + halfc, uy = (cy << sh) + halfc, uz = (cz << sh) + halfc;
-  const uint32_t b0 = warp ? b + (uint32_t)lane : b, step = warp ? 32u : 1u;
-  const bool write = !warp || lane == 0;
-  auto st = [&](int k, float v) { out[k] = v; };
-  p2m_group<P, 0, NC / 3>(px, py, pz, b0, e, step, warp, ux, uy, uz, write, st);
-  p2m_group<P, NC / 3, 2 * NC / 3>(px, py, pz, b0, e, step, warp, ux, uy, uz, write, st);
-  p2m_group<P, 2 * NC / 3, NC>(px, py, pz, b0, e, step, warp, ux, uy, uz, write, st);
+  p2m_all<P, 3>(px, py, pz, warp ? b + (uint32_t)lane : b, e, warp ? 32u : 1u, warp, lane, ux, uy,
+                uz, [&](int, int k, double v) { out[k] = (float)v; });
 }
 
 // a thread per particle j of the range (absolute index rbegin + j, key
@@ -227,28 +231,39 @@ __global__ void __launch_bounds__(256) p2m_compact_big_kernel(
       continue;
     }
     // a crowded cell: the parts that the fused pass gives its eight warps, one
-    // after another, added in the same order
-    constexpr int NC = ct2g_ncomp(P);
+    // after another, added in the same order (each lane its components, one a piece)
     uint32_t cx, cy, cz;
     demorton(key, mbits, cx, cy, cz);
     const int sh = 32 - mbits;
     const uint32_t halfc = 1u << (sh - 1);
-    double acc[NC];
+    double acc[3] = {0.0, 0.0, 0.0};
+    int at[3] = {-1, -1, -1};
+    for (uint32_t v = 0; v < 8; v++)
+      p2m_all<P, 3>(px, py, pz, b + 32u * v + (uint32_t)lane, e, 256, true, lane,
+                    (cx << sh) + halfc, (cy << sh) + halfc, (cz << sh) + halfc,
+                    [&](int piece, int k, double w) {
+                      acc[piece] += w;
+                      at[piece] = k;
+                    });
 #pragma unroll
-    for (int k = 0; k < NC; k++) acc[k] = 0.0;
-    for (int v = 0; v < 8; v++)
-      p2m_part<P>(px, py, pz, b, e, v, lane, (cx << sh) + halfc, (cy << sh) + halfc,
-                  (cz << sh) + halfc, [&](int k, double w) { acc[k] += w; });
-    if (lane == 0) {
-#pragma unroll
-      for (int k = 0; k < NC; k++) out[k] = (float)acc[k];
-    }
+    for (int q3 = 0; q3 < 3; q3++)
+      if (at[q3] >= 0) out[at[q3]] = (float)acc[q3];
   }
 }
 
 // The moments of the N cells of line `line` (x * N + y) of box `box`, from
 // the particles, into the packed smem lines sr (line l = components 2l, 2l+1
 // as .x, .y).  Ends with the block synchronised.
+// The pieces of the components: at N = 256 a thread has a cell and three pieces fit
+// the registers of 4 blocks per SM.  Shorter lines leave threads without a cell, so
+// the pieces are dealt to groups of N threads (4 pieces, 2 or 4 groups); 6 at order 6
+// for its registers.  With warp_sums and 3 blocks per SM instead of 2 at orders 5 and
+// 6: 12 boxes of a 64^3 mesh, order 5, 620 -> 447 us; one such mesh 69 -> 52; 64^3,
+// order 4, 41 -> 31; 256^3 (warp_sums alone) 1105 -> 1080.
+template <int P, int N>
+constexpr int p2m_pieces() {
+  return N >= 256 ? 3 : P <= 5 ? 4 : 6;
+}
 template <int P, int N>
 struct P2mSmem {
   uint32_t big[N];        // cells for a warp from the front, for the block from the back
@@ -267,10 +282,16 @@ __device__ __forceinline__ void p2m_line(const uint32_t *__restrict__ px,
   const int sh = 32 - mbits;
   const uint32_t halfc = 1u << (sh - 1);
   const uint32_t ux = (cx << sh) + halfc, uy = (cy << sh) + halfc;
-  for (int zc = threadIdx.x; zc < N; zc += 256) {
+  // lines of fewer cells than threads: GW threads' worth of cells, the pieces dealt
+  // to TG such groups
+  constexpr int NP = p2m_pieces<P, N>(), GW = N < 32 ? 32 : N;
+  constexpr int TG = 256 / GW < 1 ? 1 : 256 / GW < NP ? 256 / GW : NP;
+  const int tg = TG == 1 ? 0 : (int)threadIdx.x / GW;
+  for (int zc = TG == 1 ? threadIdx.x : threadIdx.x % GW; zc < N && tg < TG; zc += 256) {
     const uint32_t key = (box << (3 * mbits)) | ct2g_morton(cx, cy, (uint32_t)zc);
     const uint32_t b = cs[key], e = cs[key + 1];
     if (e - b > kWarpCell) {
+      if (tg) continue;
       if (e - b > kBlockCell)
         sm.big[N - 1 - atomicAdd(&sm.ncrowd, 1u)] = (uint32_t)zc;
       else
@@ -278,10 +299,17 @@ __device__ __forceinline__ void p2m_line(const uint32_t *__restrict__ px,
       continue;
     }
     const uint32_t uz = ((uint32_t)zc << sh) + halfc;
-    p2m_half<P, N, 0, NC / 3>(px, py, pz, b, e, 1, false, ux, uy, uz, zc, sr, true);
-    p2m_half<P, N, NC / 3, 2 * NC / 3>(px, py, pz, b, e, 1, false, ux, uy, uz, zc, sr, true);
-    p2m_half<P, N, 2 * NC / 3, NC>(px, py, pz, b, e, 1, false, ux, uy, uz, zc, sr, true);
-    if (NC & 1) sr[2 * LL::at(NL - 1, zc, 0) + 1] = 0.f;
+    each_piece(
+        [&](auto i) {
+          constexpr int I = decltype(i)::value;
+          if (I % TG == tg)
+            p2m_sum<P, I * NC / NP, (I + 1) * NC / NP>(
+                px, py, pz, b, e, 1, false, 0, ux, uy, uz, [&](int k, double v) {
+                  sr[2 * LL::at(k >> 1, zc, 0) + (k & 1)] = (float)v;
+                });
+        },
+        std::make_integer_sequence<int, NP>{});
+    if ((NC & 1) && tg == 0) sr[2 * LL::at(NL - 1, zc, 0) + 1] = 0.f;
   }
   __syncthreads();
   {  // the big cells, a warp each, then the crowded ones, a part per warp: one loop
@@ -300,13 +328,12 @@ __device__ __forceinline__ void p2m_line(const uint32_t *__restrict__ px,
         const uint32_t b = cs[key] + (uint32_t)lane + (crowd ? 32u * (uint32_t)warp : 0u),
                        e = cs[key + 1], step = crowd ? 256u : 32u;
         const uint32_t uz = (zc << sh) + halfc;
-        auto st = [&](int k, double v) {
+        auto st = [&](int, int k, double v) {
           if (crowd) sm.part[warp][k] = v;
           else sr[2 * LL::at(k >> 1, (int)zc, 0) + (k & 1)] = (float)v;
         };
-        p2m_sum<P, 0, NC / 3>(px, py, pz, b, e, step, true, ux, uy, uz, lane == 0, st);
-        p2m_sum<P, NC / 3, 2 * NC / 3>(px, py, pz, b, e, step, true, ux, uy, uz, lane == 0, st);
-        p2m_sum<P, 2 * NC / 3, NC>(px, py, pz, b, e, step, true, ux, uy, uz, lane == 0, st);
+        p2m_all<P, (N < 256 && P > 4) ? NP : 3>(px, py, pz, b, e, step, true, lane, ux, uy, uz,
+                                                st);
         if ((NC & 1) && lane == 0 && !crowd) sr[2 * LL::at(NL - 1, (int)zc, 0) + 1] = 0.f;
       }
       if (crowd) {  // the parts added in order
@@ -381,10 +408,11 @@ __device__ __forceinline__ void store_half_spectra(const float2 *s, float2 *rows
   }
 }
 
-// occupancy: 4 blocks per SM up to order 4 (64 registers); at N = 512 the
+// occupancy: 4 blocks per SM up to order 4 (64 registers), 3 beyond on short lines
+// (2 where the lines fill the shared memory); at N = 512 the
 // 32-point in-register DFTs need more registers than that, so 2
 template <int P, int N, int SRC>
-__global__ void __launch_bounds__(256, N >= 512 ? 2 : P <= 4 ? 4 : 2) fftz_p2m_r2c_kernel(
+__global__ void __launch_bounds__(256, N >= 512 ? 2 : P <= 4 ? 4 : N <= 128 ? 3 : 2) fftz_p2m_r2c_kernel(
     const uint32_t *__restrict__ px, const uint32_t *__restrict__ py,
     const uint32_t *__restrict__ pz, const uint32_t *__restrict__ cs, int mbits,
     float *__restrict__ grid, int64_t CB, float2 *__restrict__ spec, int ldk,

@@ -53,3 +53,31 @@ def test_crowded_cell_moments(gpu, n):
         g.close()
     scale = np.sqrt(np.mean(np.sum(f[0] ** 2, 1)))
     assert np.abs(f[0] - f[1]).max() <= 1e-5 * scale
+
+
+@pytest.mark.parametrize("mesh,p", [(8, 1), (8, 6), (16, 2), (16, 5), (32, 3), (32, 6), (64, 1), (64, 4),
+                                    (64, 5), (64, 6), (128, 2), (128, 4), (128, 5), (128, 6)])
+def test_line_moments(gpu, mesh, p):
+    """Cells of 1 .. 6 particles (a thread each, the components dealt to the line's
+    thread groups), 7 .. 40 (a warp) and 300 (the block) along two lines, against the
+    moment grid's: as above, one FP32 rounding of the moments apart."""
+    rng = np.random.default_rng(mesh + p)
+    pos = []
+    for z, n in zip((0, 1, 3, 4, mesh // 2, mesh - 2, mesh - 1), (1, 6, 7, 40, 300, 2, 33)):
+        for line in ((2, 3), (mesh - 1, 0)):
+            c = (np.array([line[0], line[1], z]) + 0.5) / mesh
+            pos.append(c + rng.uniform(-0.45, 0.45, (n, 3)) / mesh)
+    pos = np.concatenate(pos)
+    P = ics._pack(pos, len(pos))
+    f = []
+    for grid in (True, False):
+        g = Gravity(mesh=mesh, order=p, bwidth=1.0, hsoft=0.5 / mesh, GM=1.0 / len(pos))
+        g.upload_dict(P)
+        g.particle_to_grid()
+        if grid:
+            g.compute_multipoles()
+        g.compute_forces()
+        f.append(g.forces()[0])
+        g.close()
+    scale = np.sqrt(np.mean(np.sum(f[0] ** 2, 1)))
+    assert np.abs(f[0] - f[1]).max() <= 1e-5 * scale
