@@ -170,9 +170,23 @@ struct NearArgs {
 // (50 k particles, mesh 64), 2.75 / 2.82 / 2.96 / 2.96 (262 k, 128, with the learned
 // correction), 11.9 / 11.75 / 11.58 / 11.52 (2.1 M, 256).
 uint32_t heavy_min(int M) { return M <= 128 ? 1024u : 8192u; }
+// SPLIT: the sparse sinks of the sphere kernel.  A coordinate in the frame of a
+// 4-cell block has lost up to three bits of the offset from its own cell's centre, so that
+// the separation of two particles of one cell was off by up to 4 ulp of a
+// cell (forces 1e-6 to 3e-6 rms off where the cell-by-cell form is 1e-7); so sinks and sources
+// keep offset and cell centre apart, and a separation is (offset - offset) + (centre - centre):
+// exact inside a cell, rounded at the size of a cell and of itself beyond.  Two
+// more packed additions and half a broadcast load per coordinate and pair.  (The dense
+// chunks' frame is the sink cell itself, where the pairs of the cell are exact as they are;
+// the Plummer kernel's sparse sinks are staged in the block's frame.)
+template <int KERNEL, bool SPARSE>
+constexpr bool kSplit = KERNEL == CT2G_SOFT_SPHERE && SPARSE;
 // floats of staging per warp: two batches (x, y, z and cell bits of 32
-// sources), then the window's table
-constexpr int kBatch = 128, kStage = 2 * kBatch + 128;
+// sources; SPLIT: their cells' centres), then the window's table
+template <bool SPLIT>
+constexpr int kBatch = SPLIT ? 224 : 128;
+template <bool SPLIT>
+constexpr int kStage = 2 * kBatch<SPLIT> + 128;
 // a coordinate that makes r^2 infinite: an empty slot of the last batch adds 0
 constexpr float kFar = 3e19f;
 
@@ -219,10 +233,10 @@ __device__ __forceinline__ void pair_weights(f32x2 dx, f32x2 dy, f32x2 dz, f32x2
   }
 }
 
-// a lane's sink (coordinates in both halves) and its packed sums +d g, +1/r
-// (the caller negates)
+// a lane's sink (coordinates in both halves; SPLIT: its offset, and its cell's
+// centre in CX, CY, CZ) and its packed sums +d g, +1/r (the caller negates)
 struct Sink {
-  f32x2 X, Y, Z, ax, ay, az, ap;
+  f32x2 X, Y, Z, ax, ay, az, ap, CX, CY, CZ;
 };
 
 // interactions of NS sinks with the four sources of quad qd (negated
@@ -244,11 +258,25 @@ __device__ __forceinline__ void quad_term(const float *sb, int qd, uint32_t bits
   const f32x2 px[2] = {f2_pack(x.x, x.y), f2_pack(x.z, x.w)};
   const f32x2 py[2] = {f2_pack(y.x, y.y), f2_pack(y.z, y.w)};
   const f32x2 pz[2] = {f2_pack(z.x, z.y), f2_pack(z.z, z.w)};
+  f32x2 cx[2], cy[2], cz[2];
+  if constexpr (kSplit<KERNEL, MASKED>) {
+    const float4 a = reinterpret_cast<const float4 *>(sb + 128)[qd];
+    const float4 b = reinterpret_cast<const float4 *>(sb + 160)[qd];
+    const float4 c = reinterpret_cast<const float4 *>(sb + 192)[qd];
+    cx[0] = f2_pack(a.x, a.y), cx[1] = f2_pack(a.z, a.w);
+    cy[0] = f2_pack(b.x, b.y), cy[1] = f2_pack(b.z, b.w);
+    cz[0] = f2_pack(c.x, c.y), cz[1] = f2_pack(c.z, c.w);
+  }
 #pragma unroll
   for (int h = 0; h < 2; h++)
 #pragma unroll
     for (int u = 0; u < NS; u++) {
-      const f32x2 dx = f2_add(k[u].X, px[h]), dy = f2_add(k[u].Y, py[h]), dz = f2_add(k[u].Z, pz[h]);
+      f32x2 dx = f2_add(k[u].X, px[h]), dy = f2_add(k[u].Y, py[h]), dz = f2_add(k[u].Z, pz[h]);
+      if constexpr (kSplit<KERNEL, MASKED>) {
+        dx = f2_add(dx, f2_add(k[u].CX, cx[h]));
+        dy = f2_add(dy, f2_add(k[u].CY, cy[h]));
+        dz = f2_add(dz, f2_add(k[u].CZ, cz[h]));
+      }
       f32x2 g, pp;
       pair_weights<KERNEL, POT, MASKED>(dx, dy, dz, H2, h2, hinv, hinv3, on[2 * h], on[2 * h + 1],
                                         g, pp);
@@ -312,15 +340,18 @@ struct Chunk {
     const uint32_t w = word ? A.cs[(size_t)(nblk + 1) << 6] - A.cs[(size_t)nblk << 6] : 0u;
     return __reduce_add_sync(0xffffffffu, w);
   }
+  template <bool SPLIT>
   __device__ __forceinline__ void sinks(const NearArgs &A, float hc, Sink (&k)[NS]) const {
     int ix, iy, iz;
     inblock((int)p, ix, iy, iz);
+    const float cx = (float)(ix - fx) * hc, cy = (float)(iy - fy) * hc, cz = (float)(iz - fz) * hc;
 #pragma unroll
     for (int u = 0; u < NS; u++) {
       const float4 q = A.src[idx[u]];
-      const float sx = fmaf((float)(ix - fx), hc, q.x), sy = fmaf((float)(iy - fy), hc, q.y),
-                  sz = fmaf((float)(iz - fz), hc, q.z);
-      k[u] = Sink{f2_pack(sx, sx), f2_pack(sy, sy), f2_pack(sz, sz), 0ull, 0ull, 0ull, 0ull};
+      const float sx = SPLIT ? q.x : cx + q.x, sy = SPLIT ? q.y : cy + q.y,
+                  sz = SPLIT ? q.z : cz + q.z;
+      k[u] = Sink{f2_pack(sx, sx), f2_pack(sy, sy), f2_pack(sz, sz), 0ull, 0ull, 0ull, 0ull,
+                  f2_pack(cx, cx), f2_pack(cy, cy), f2_pack(cz, cz)};
     }
   }
   // The window of candidate cells w0 ..: its table (a cell per lane: its centre
@@ -397,13 +428,18 @@ __device__ __forceinline__ uint32_t stream_slot(uint32_t excl, uint32_t b, uint3
 
 // a fetched source (offset q from its cell's centre, slot t of the window) into
 // a staged batch; off: an empty slot
-template <bool SPARSE>
+template <bool SPARSE, bool SPLIT>
 __device__ __forceinline__ void stage_source(float *sb, const float4 &w, const float4 &q,
                                              uint32_t t, bool on, int lane) {
-  sb[lane] = on ? w.x - q.x : kFar;
-  sb[32 + lane] = w.y - q.y;
-  sb[64 + lane] = w.z - q.z;
+  sb[lane] = !on ? kFar : SPLIT ? -q.x : w.x - q.x;
+  sb[32 + lane] = SPLIT ? -q.y : w.y - q.y;
+  sb[64 + lane] = SPLIT ? -q.z : w.z - q.z;
   if (SPARSE) sb[96 + lane] = __uint_as_float(on ? 1u << t : 0u);
+  if (SPLIT) {
+    sb[128 + lane] = w.x;
+    sb[160 + lane] = w.y;
+    sb[192 + lane] = w.z;
+  }
 }
 
 struct Soft {
@@ -490,16 +526,17 @@ __device__ __forceinline__ void group_sync(int S, int group) {
 template <int KERNEL, bool POT>
 __device__ __forceinline__ bool sparse_chunk(const NearArgs &A, const uint2 cd, int s, int S,
                                              int group, float *stage, int lane) {
+  constexpr bool SPLIT = kSplit<KERNEL, true>;
   Chunk<true, 1> k;
   k.open(A, cd, lane);
   if (k.sources(A) > A.heavy_min) return false;
   const float hc = 1.0f / (float)(1 << A.mbits);
   Sink sink[1];
-  k.sinks(A, hc, sink);
+  k.template sinks<SPLIT>(A, hc, sink);
   const Soft soft(A.soft);
   float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
   uint32_t nsrc = 0;
-  float4 *win = reinterpret_cast<float4 *>(stage + 2 * kBatch);
+  float4 *win = reinterpret_cast<float4 *>(stage + 2 * kBatch<SPLIT>);
   for (uint32_t r0 = 0; r0 < k.C; r0 += 32u * (uint32_t)S) {
     const uint32_t w0 = r0 + 32u * (uint32_t)s;
     if (w0 < k.C) {
@@ -516,11 +553,11 @@ __device__ __forceinline__ bool sparse_chunk(const NearArgs &A, const uint2 cd, 
       float *sb = stage;
       if (total) fetch(0u);
       for (uint32_t b = 0; b < total; b += 32u) {
-        stage_source<true>(sb, win[t], nq, t, b + (uint32_t)lane < total, lane);
+        stage_source<true, SPLIT>(sb, win[t], nq, t, b + (uint32_t)lane < total, lane);
         __syncwarp();
         if (b + 32u < total) fetch(b + 32u);
         eval_batch<KERNEL, POT, true, 1>(sb, total - b, bits, sink, soft);
-        sb = sb == stage ? stage + kBatch : stage;
+        sb = sb == stage ? stage + kBatch<SPLIT> : stage;
       }
     }
     const float4 v = take<POT>(sink[0]);
@@ -533,7 +570,7 @@ __device__ __forceinline__ bool sparse_chunk(const NearArgs &A, const uint2 cd, 
       if (s == 0) {
         add(tot, v);
         const int nw = (int)min((uint32_t)S, (k.C - r0 + 31u) / 32u);
-        for (int u = 1; u < nw; u++) add(tot, reinterpret_cast<const float4 *>(stage + u * kStage)[lane]);
+        for (int u = 1; u < nw; u++) add(tot, reinterpret_cast<const float4 *>(stage + u * kStage<SPLIT>)[lane]);
       }
       group_sync(S, group);
     }
@@ -553,7 +590,8 @@ __device__ __forceinline__ bool sparse_chunk(const NearArgs &A, const uint2 cd, 
 // do not depend on S.
 template <int KERNEL, bool POT>
 __global__ void __launch_bounds__(256, 4) near_sparse_kernel(const NearArgs A) {
-  __shared__ __align__(16) float stage[8 * kStage];
+  constexpr int ST = kStage<kSplit<KERNEL, true>>;
+  __shared__ __align__(16) float stage[8 * ST];
   __shared__ uint32_t taken_s[2][8];  // by the parity of the turn: one barrier a turn
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t nch = *A.nsparse;
@@ -574,7 +612,7 @@ __global__ void __launch_bounds__(256, 4) near_sparse_kernel(const NearArgs A) {
       ch = __shfl_sync(0xffffffffu, ch, 0);
     }
     if (ch >= nch) break;
-    if (!sparse_chunk<KERNEL, POT>(A, list[ch], s, S, group, stage + wib * kStage, lane) &&
+    if (!sparse_chunk<KERNEL, POT>(A, list[ch], s, S, group, stage + wib * ST, lane) &&
         s == 0 && lane == 0)
       A.heavy[atomicAdd(A.work + 1, 1u)] = ch;
   }
@@ -588,21 +626,23 @@ __global__ void __launch_bounds__(256, 4) near_sparse_kernel(const NearArgs A) {
 // launch half idle).  NS sinks per lane: a dense chunk of more than 32 sinks
 // holds two, so that each staged quad feeds eight interactions.
 constexpr uint32_t kSeg = 256;
+template <int KERNEL>
 struct CoopSmem {
-  float stage[8][2 * kBatch];
+  float stage[8][2 * kBatch<kSplit<KERNEL, true>>];
   float4 win[8][32];
   uint32_t excl[8][32], bits[8][32], total[8];
   uint32_t chunk[2];
 };
 
 template <int KERNEL, bool POT, bool SPARSE, int NS>
-__device__ __forceinline__ void coop_chunk(const NearArgs &A, const uint2 cd, CoopSmem &sm,
-                                           int wib, int lane) {
+__device__ __forceinline__ void coop_chunk(const NearArgs &A, const uint2 cd,
+                                           CoopSmem<KERNEL> &sm, int wib, int lane) {
+  constexpr bool SPLIT = kSplit<KERNEL, SPARSE>;
   Chunk<SPARSE, NS> k;
   k.open(A, cd, lane);
   const float hc = 1.0f / (float)(1 << A.mbits);
   Sink sink[NS];
-  k.sinks(A, hc, sink);
+  k.template sinks<SPLIT>(A, hc, sink);
   const Soft soft(A.soft);
   uint32_t nsrc = 0;
   for (uint32_t r0 = 0; r0 < k.C; r0 += 256u) {
@@ -646,7 +686,7 @@ __device__ __forceinline__ void coop_chunk(const NearArgs &A, const uint2 cd, Co
     if (w < 8) fetch();
     __syncwarp();  // the last batch of the round before is read
     while (w < 8) {
-      stage_source<SPARSE>(sb, sm.win[w][t], nq, t, b + (uint32_t)lane < tot, lane);
+      stage_source<SPARSE, SPLIT>(sb, sm.win[w][t], nq, t, b + (uint32_t)lane < tot, lane);
       __syncwarp();
       const uint32_t n = tot - b, eb = bits;
       b += 32u;
@@ -657,7 +697,7 @@ __device__ __forceinline__ void coop_chunk(const NearArgs &A, const uint2 cd, Co
       }
       if (w < 8) fetch();
       eval_batch<KERNEL, POT, SPARSE, NS>(sb, n, eb, sink, soft);
-      sb = sb == sm.stage[wib] ? sm.stage[wib] + kBatch : sm.stage[wib];
+      sb = sb == sm.stage[wib] ? sm.stage[wib] + kBatch<SPLIT> : sm.stage[wib];
     }
   }
   // the eight warps' sums, in order
@@ -685,7 +725,7 @@ __device__ __forceinline__ void coop_chunk(const NearArgs &A, const uint2 cd, Co
 
 template <int KERNEL, bool POT>
 __global__ void __launch_bounds__(256, 3) near_coop_kernel(const NearArgs A) {
-  __shared__ __align__(16) CoopSmem sm;
+  __shared__ __align__(16) CoopSmem<KERNEL> sm;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t nh = A.nsparse ? A.work[1] : 0u, nch = nh + *A.ndense;
   if (threadIdx.x == 0) sm.chunk[0] = atomicAdd(A.work + 2, 1u);
