@@ -440,7 +440,7 @@ int ct2g_create_boxes(const ct2g_options *opt, int nbox, ct2g_ctx **out) {
     if ((rc = ct2g_fft_init(ctx)) != CT2G_OK) break;
     // near-field stencil: integer offsets |o|^2 <= bwidth^2 (the fixed form
     // of particle_cell_neighbors, src/particle.cpp:302-318), as bit masks
-    const double bw2 = (double)opt->bwidth * (double)opt->bwidth;
+    const int bw2 = ct2g_radius2(opt->bwidth);
     // stencil bits per (in-block Morton position p, block offset (dX,dY,dZ)):
     // cells b of the neighbouring 4x4x4 block with |4 d + pos(b) - pos(p)|^2 <= bwidth^2
     {
@@ -459,7 +459,7 @@ int ct2g_create_boxes(const ct2g_options *opt, int nbox, ct2g_ctx **out) {
             int bx, by, bz;
             pos(b, bx, by, bz);
             const int ox = 4 * dX + bx - px, oy = 4 * dY + by - py, oz = 4 * dZ + bz - pz;
-            if ((double)(ox * ox + oy * oy + oz * oz) <= bw2) m[p * 27 + o] |= 1ull << b;
+            if (ox * ox + oy * oy + oz * oz <= bw2) m[p * 27 + o] |= 1ull << b;
           }
         }
       }

@@ -396,6 +396,10 @@ int ct2g_fft_cols_tc(ct2g_ctx *ctx, float2 *spec, int N, size_t nouter, size_t o
 int ct2g_learned_apply(ct2g_ctx *ctx, bool pot);
 int ct2g_learned_resize(ct2g_ctx *ctx);  // per-cell arrays follow the particle capacity
 void ct2g_learned_free(ct2g_ctx *ctx);
+// The largest whole |o|^2 within the stencil radius bw.  Squared in FP64: float(sqrt(3))
+// squared is just below 3, and rounded to FP32 it is 3; the masks, the Green's
+// table and the kernels' lanes must agree on which cells that leaves to the mesh.
+inline int ct2g_radius2(float bw) { return (int)std::floor((double)bw * (double)bw); }
 // widened near-field sums of selected cells (ct2g_near.cu): dense-style chunks
 // (<= 32 consecutive sinks of one cell, (first particle, count), *nd of them)
 // over the stencil masks stm, sparse-style ones (*ns, their sinks in slist)
@@ -403,7 +407,7 @@ void ct2g_learned_free(ct2g_ctx *ctx);
 // counters, zero on entry
 int ct2g_near_window(ct2g_ctx *ctx, const uint2 *dch, const uint32_t *nd, const uint2 *sch,
                      const uint32_t *ns, const uint32_t *slist, uint32_t *work,
-                     const unsigned long long *stm, float lo2, float hi2, bool pot, float *fx,
+                     const unsigned long long *stm, int lo2, int hi2, bool pot, float *fx,
                      float *fy, float *fz, float *po);
 // D^n phi_eps(-o h) for the offsets o (x,y,z triples) -> d_out[nshell][nc]
 int ct2g_shell_greens(ct2g_ctx *ctx, const std::vector<int> &offs3, float *d_out);

@@ -1195,9 +1195,9 @@ int widen_block_p(ct2g_ctx *ctx, bool pot, float *fx, float *fy, float *fz, floa
       L->d_cnt, L->sel_cells, L->cells, L->mc, L->idx, geo_of(ctx), L->d_shell, L->d_shellG,
       L->nshell, L->lsub);
   CT2G_LAUNCHED(ctx);
-  const float bw = ctx->opt.bwidth, bx = L->bw_ext;
   CT2G_TRY(ct2g_near_window(ctx, L->dchunks, L->d_cnt + 5, L->chunks, L->d_cnt + 2, L->ssink2,
-                            L->d_cnt + 8, L->d_stm, bw * bw, bx * bx, pot, fx, fy, fz, po));
+                            L->d_cnt + 8, L->d_stm, ct2g_radius2(ctx->opt.bwidth),
+                            ct2g_radius2(L->bw_ext), pot, fx, fy, fz, po));
   if (pot)
     shell_l2p_kernel<P, true><<<G, T, 0, st>>>(L->d_cnt, L->ssink, L->scell, ctx->keys, begin,
                                                 ctx->mbits, ctx->src, L->lsub, ctx->box_gm, fx, fy,
@@ -1333,11 +1333,11 @@ int ct2g_learned_enable(ct2g_ctx *ctx, float bwidth_ext) {
   // shell offsets, nearest first, and three distance bins of equal size
   std::vector<std::array<int, 3>> offs;
   const int B = (int)std::floor(bwidth_ext);
-  const double b2 = (double)bw * bw, x2 = (double)bwidth_ext * bwidth_ext;
+  const int b2 = ct2g_radius2(bw), x2 = ct2g_radius2(bwidth_ext);
   for (int i = -B; i <= B; i++)
     for (int j = -B; j <= B; j++)
       for (int k = -B; k <= B; k++) {
-        const double d2 = (double)(i * i + j * j + k * k);
+        const int d2 = i * i + j * j + k * k;
         if (d2 > b2 && d2 <= x2) offs.push_back({i, j, k});
       }
   std::stable_sort(offs.begin(), offs.end(), [](const std::array<int, 3> &a, const std::array<int, 3> &b) {
@@ -1378,7 +1378,7 @@ int ct2g_learned_enable(ct2g_ctx *ctx, float bwidth_ext) {
           pos(b, bx, by, bz);
           const int ox = 4 * (o / 9 - 1) + bx - px, oy = 4 * ((o / 3) % 3 - 1) + by - py,
                     oz = 4 * (o % 3 - 1) + bz - pz;
-          const double d2 = (double)(ox * ox + oy * oy + oz * oz);
+          const int d2 = ox * ox + oy * oy + oz * oz;
           if (d2 > b2 && d2 <= x2) m[p * 27 + o] |= 1ull << b;
         }
     }

@@ -196,7 +196,7 @@ __device__ __forceinline__ double ipow(double x, int e) {
 }
 
 // real-space part for components [k0, k0+K) at every lattice offset
-__global__ void greens_real_kernel(int mbits, int p, int kernel, double soft, double bw2,
+__global__ void greens_real_kernel(int mbits, int p, int kernel, double soft, int bw2,
                                    double alpha, const DTerm *__restrict__ terms,
                                    const int *__restrict__ nterms, int k0, int K,
                                    double *__restrict__ out) {
@@ -210,7 +210,7 @@ __global__ void greens_real_kernel(int mbits, int p, int kernel, double soft, do
   const double h = 1.0 / M;
   const double R[3] = {o[0] * h, o[1] * h, o[2] * h};
   const double r2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
-  const bool near = (double)(o[0] * o[0] + o[1] * o[1] + o[2] * o[2]) <= bw2;
+  const bool near = o[0] * o[0] + o[1] * o[1] + o[2] * o[2] <= bw2;
   double fe[CT2G_MAX_ORDER + 1], fk[CT2G_MAX_ORDER + 1], f[CT2G_MAX_ORDER + 1];
   radial_erf(r2, alpha, p, fe);
   if (!near) {
@@ -450,7 +450,7 @@ int ct2g_build_greens(ct2g_ctx *ctx) {
                     ctx->stream);
     cudaMemcpyAsync(d_mi, mi.data(), sizeof(int) * 3 * nc, cudaMemcpyHostToDevice, ctx->stream);
     const double soft = ctx->opt.hsoft;
-    const double bw2 = (double)ctx->opt.bwidth * (double)ctx->opt.bwidth;
+    const int bw2 = ct2g_radius2(ctx->opt.bwidth);
     for (int k0 = 0; k0 < nc && rc == CT2G_OK; k0 += K) {
       const int kk = std::min(K, nc - k0);
       greens_real_kernel<<<ct2g_div_up(ctx->C, 128), 128, 0, ctx->stream>>>(

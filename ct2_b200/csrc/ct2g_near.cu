@@ -1003,7 +1003,7 @@ Walk make_walk(int mbits) {
   return w;
 }
 
-NearArgs near_args(ct2g_ctx *ctx, const unsigned long long *stm, float lo2, float hi2, float *fx,
+NearArgs near_args(ct2g_ctx *ctx, const unsigned long long *stm, int lo2, int hi2, float *fx,
                    float *fy, float *fz, float *pot, bool store) {
   NearArgs A{};
   A.cs = ctx->cell_start;
@@ -1015,9 +1015,8 @@ NearArgs near_args(ct2g_ctx *ctx, const unsigned long long *stm, float lo2, floa
   A.src = ctx->src;
   A.mbits = ctx->mbits;
   A.soft = ctx->opt.hsoft;
-  // integers d2 with lo2 < d2 <= hi2
-  A.lo2 = (int)std::floor(lo2);
-  A.hi2 = (int)std::floor(hi2);
+  A.lo2 = lo2;
+  A.hi2 = hi2;
   A.box_gm = ctx->box_gm;
   A.ofx = fx;
   A.ofy = fy;
@@ -1083,8 +1082,7 @@ template <int K, bool POT>
 int launch_near(ct2g_ctx *ctx, cudaStream_t st, float *fx, float *fy, float *fz, float *pot,
                 bool store) {
   uint32_t *c = ctx->d_counts;
-  NearArgs A = near_args(ctx, ctx->stmask, -1.f, ctx->opt.bwidth * ctx->opt.bwidth, fx, fy, fz, pot,
-                         store);
+  NearArgs A = near_args(ctx, ctx->stmask, -1, ct2g_radius2(ctx->opt.bwidth), fx, fy, fz, pot, store);
   A.dchunks = ctx->chunks;
   A.schunks = ctx->schunks;
   A.ndense = c;
@@ -1136,7 +1134,7 @@ __global__ void combine_kernel(size_t b, size_t n, float *__restrict__ fx, float
 // added into the given force buffers; work: four zeroed counters
 int ct2g_near_window(ct2g_ctx *ctx, const uint2 *dch, const uint32_t *nd, const uint2 *sch,
                      const uint32_t *ns, const uint32_t *slist, uint32_t *work,
-                     const unsigned long long *stm, float lo2, float hi2, bool pot, float *fx,
+                     const unsigned long long *stm, int lo2, int hi2, bool pot, float *fx,
                      float *fy, float *fz, float *po) {
   NearArgs A = near_args(ctx, stm, lo2, hi2, fx, fy, fz, po, false);
   A.dchunks = dch;
