@@ -1014,6 +1014,10 @@ int ct2g_fft3d_f32_dev(ct2g_ctx *ctx, int dir, void *d_real, void *d_complex, in
   CT2G_TRY(check(ctx));
   if (!d_real || !d_complex || batch < 1 || !is_pow2(N) || N < 4 || N > 512)
     return ct2g_fail(ctx, CT2G_EINVAL, "fft3d_f32_dev: bad arguments");
+  // the z passes move the real grid in 16-byte pieces
+  if (((uintptr_t)d_real & 15) != 0 || ((uintptr_t)d_complex & 7) != 0)
+    return ct2g_fail(ctx, CT2G_EINVAL,
+                     "fft3d_f32_dev: the real grid must be 16-byte, the spectrum 8-byte aligned");
   if (dir > 0)
     return ct2g_fft_r2c_f32(ctx, (const float *)d_real, (float2 *)d_complex, N, batch, N / 2 + 1);
   return ct2g_fft_c2r_f32(ctx, (float2 *)d_complex, (float *)d_real, N, batch, N / 2 + 1);

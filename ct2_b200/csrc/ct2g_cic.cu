@@ -72,6 +72,8 @@ extern "C" int ct2g_cic_deposit(ct2g_ctx *ctx, int N, void *d_grid) {
   CT2G_TRY(ct2g_check(ctx));
   if (!d_grid || !pow2(N) || N < 4 || N > 512)
     return ct2g_fail(ctx, CT2G_EINVAL, "cic_deposit: N a power of two in [4, 512], grid non-null");
+  if (((uintptr_t)d_grid & 3) != 0)
+    return ct2g_fail(ctx, CT2G_EINVAL, "cic_deposit: the grid must be 4-byte aligned");
   if (!ctx->has_particles) return ct2g_fail(ctx, CT2G_ESTATE, "no particles uploaded");
   const size_t N3 = (size_t)N * N * N;
   float2 *g = reinterpret_cast<float2 *>(d_grid);

@@ -431,7 +431,9 @@ int ct2g_twiddles(ct2g_ctx *ctx, int which, int N, double *out);
  * its own makes the context's stream wait for that stream first (an event)
  * and its own stream wait for the context's afterwards. */
 /* FP32 device-pointer variant on the context stream, interleaved complex
- * output (float2[batch][N][N][N/2+1]); dir = +1 forward r2c, -1 inverse c2r */
+ * output (float2[batch][N][N][N/2+1]); dir = +1 forward r2c, -1 inverse c2r.
+ * N: power of two, 4..512; the real grid 16-byte aligned, the spectrum 8-byte
+ * (CT2G_EINVAL otherwise). */
 int ct2g_fft3d_f32_dev(ct2g_ctx *ctx, int dir, void *d_real, void *d_complex, int N,
                        int batch);
 /* Complex-to-complex 3D FFT of `batch` device grids float2[batch][N][N][N]
@@ -446,7 +448,8 @@ int ct2g_fft3d_c2c_f32_dev(ct2g_ctx *ctx, int dir, void *d_data, int N, int batc
  * the CIC mass and the three first moments about each mesh point (offsets in
  * mesh units), the imaginary parts zero.  A particle at x lies between mesh
  * points floor(xN - 1/2) and the next, with linear weights per axis.  No
- * counterpart in the reference. */
+ * counterpart in the reference.  The grid 4-byte aligned; on a 16-byte boundary
+ * the deposit takes half of its atomic additions in pairs. */
 int ct2g_cic_deposit(ct2g_ctx *ctx, int N, void *d_grid);
 
 /* FP64 Ewald direct sum over ALL particles of the context as sources, at the
