@@ -194,6 +194,9 @@ int replay(ct2g_batch *b, int *max_rung) {
   for (size_t i = 0; i < b->ctx.size(); i++) {
     ct2g_ctx *c = b->ctx[i];
     c->launches += b->launches[i];
+    // as the eager step leaves it: the particles have moved
+    c->grid_valid = c->moments_valid = c->expansions_valid = c->forces_valid = false;
+    c->pot_valid = false;
     if (c->stream != b->s0) CT2G_CUDA(c0, cudaStreamWaitEvent(c->stream, b->t1, 0));
   }
   b->launched = true;
