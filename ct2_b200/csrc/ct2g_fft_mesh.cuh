@@ -1062,7 +1062,9 @@ __device__ __forceinline__ void cols_step2(const float2 *s, ST st, int off = 0) 
 // max(N, 32) threads by the degree of a, so that every thread has work: with a
 // thread per row, 64 of 256 did order 5's 462 complex terms each (fused x pass
 // of twelve boxes at mesh 64, order 5: 842 -> 475 us, with the odd row pitch).  A group reads what its
-// outputs need, and all groups write after a barrier.
+// outputs need, and all groups write after the block's one barrier, which stands outside
+// their branches; so that the registers across it are the largest group's and not all the
+// outputs', each keeps output A as its rank(A)-th.
 template <int P>
 struct Mg2lSplit {
   static constexpr MiTable<P> mi{};
@@ -1071,38 +1073,52 @@ struct Mg2lSplit {
   static constexpr int group(int d, int NG) {
     if (NG == 4) return d <= 3 ? d : d == 4 ? 0 : d == 5 ? 3 : 1;
     if (P <= 3) return d & 1;
-    if (P == 6) return d >= 3;
+    if (P == 6) return d >= 3 && d <= 5;  // (434 of 924 terms, and 46 outputs of 84)
     return d == 2 || d == 3 || d == 5;
   }
+  static constexpr int of(int a, int NG) { return group(mi.deg[a], NG); }
+  // outputs of a's group before a, and the outputs of the largest group
+  static constexpr int rank(int a, int NG) {
+    int r = 0;
+    for (int b = 0; b < a; b++) r += of(b, NG) == of(a, NG);
+    return r;
+  }
+  static constexpr int most(int NG) {
+    int m = 0;
+    for (int a = 0; a < ct2g_ncomp(P); a++) m = rank(a, NG) >= m ? rank(a, NG) + 1 : m;
+    return m;
+  }
 };
-template <int P, int GS, int NG, int G, int I>
-__device__ __forceinline__ void mg2l_group_term(const float2 *m, const float *g, float2 (&L)[ct2g_ncomp(P)]) {
+template <int P, int GS, int NG, int G, int I, int K>
+__device__ __forceinline__ void mg2l_group_term(const float2 *m, const float *g, float2 (&L)[K]) {
   constexpr int A = Mg2lTab<P>::t.a[I], B = Mg2lTab<P>::t.b[I], AB = Mg2lTab<P>::t.ab[I];
-  if constexpr (Mg2lSplit<P>::group(Mg2lSplit<P>::mi.deg[A], NG) == G) {
-    if constexpr (Mg2lTab<P>::t.first[I] != 0) L[A] = make_float2(0.f, 0.f);
+  if constexpr (Mg2lSplit<P>::of(A, NG) == G) {
+    constexpr int R = Mg2lSplit<P>::rank(A, NG);
+    if constexpr (Mg2lTab<P>::t.first[I] != 0) L[R] = make_float2(0.f, 0.f);
     const float gv = g[AB * GS];
     const float2 mb = m[B];
     if constexpr (Mg2lTab<P>::t.odd[I] == 0) {
-      L[A].x = fmaf(gv, mb.x, L[A].x);
-      L[A].y = fmaf(gv, mb.y, L[A].y);
+      L[R].x = fmaf(gv, mb.x, L[R].x);
+      L[R].y = fmaf(gv, mb.y, L[R].y);
     } else {  // i*g*(mx + i my) = (-g my, g mx)
-      L[A].x = fmaf(-gv, mb.y, L[A].x);
-      L[A].y = fmaf(gv, mb.x, L[A].y);
+      L[R].x = fmaf(-gv, mb.y, L[R].x);
+      L[R].y = fmaf(gv, mb.x, L[R].y);
     }
   }
 }
-template <int P, int NG, int G, int A>
-__device__ __forceinline__ void mg2l_group_store(float2 *row, const float2 (&L)[ct2g_ncomp(P)]) {
-  if constexpr (Mg2lSplit<P>::group(Mg2lSplit<P>::mi.deg[A], NG) == G) row[A] = L[A];
+template <int P, int GS, int NG, int G, int K, int... I>
+__device__ __forceinline__ void mg2l_group_sums(const float2 *m, const float *g, float2 (&L)[K],
+                                                std::integer_sequence<int, I...>) {
+  (mg2l_group_term<P, GS, NG, G, I>(m, g, L), ...);
 }
-template <int P, int GS, int NG, int G, int... I, int... A>
-__device__ __forceinline__ void mg2l_group(float2 *row, const float *g, bool on,
-                                           std::integer_sequence<int, I...>,
-                                           std::integer_sequence<int, A...>) {
-  float2 L[ct2g_ncomp(P)];
-  if (on) (mg2l_group_term<P, GS, NG, G, I>(row, g, L), ...);
-  __syncthreads();
-  if (on) (mg2l_group_store<P, NG, G, A>(row, L), ...);
+template <int P, int NG, int G, int A, int K>
+__device__ __forceinline__ void mg2l_group_put(float2 *row, const float2 (&L)[K]) {
+  if constexpr (Mg2lSplit<P>::of(A, NG) == G) row[A] = L[Mg2lSplit<P>::rank(A, NG)];
+}
+template <int P, int NG, int G, int K, int... A>
+__device__ __forceinline__ void mg2l_group_store(float2 *row, const float2 (&L)[K],
+                                                 std::integer_sequence<int, A...>) {
+  (mg2l_group_put<P, NG, G, A>(row, L), ...);
 }
 template <int P, int N, int PITCH, bool GREG, int GS>
 __device__ __forceinline__ void contract_column(float2 *s, int off, const float *g) {
@@ -1126,16 +1142,20 @@ __device__ __forceinline__ void contract_column(float2 *s, int off, const float 
     }
   } else {
     const int qi = threadIdx.x % TG, gr = threadIdx.x / TG;
-    const bool on = qi < N;
+    const int G = qi < N ? gr : NG;  // (threads past the rows or the groups: none)
     float2 *row = s + qi * PITCH + off;
     const std::make_integer_sequence<int, NP> I{};
     const std::make_integer_sequence<int, NC> A{};
-    // (each branch holds the block's one barrier; threads past the groups only wait)
-    if (gr == 0) mg2l_group<P, GS, NG, 0>(row, g + qi, on, I, A);
-    else if (gr == 1) mg2l_group<P, GS, NG, 1>(row, g + qi, on, I, A);
-    else if (NG == 4 && gr == 2) mg2l_group<P, GS, NG, NG == 4 ? 2 : 0>(row, g + qi, on, I, A);
-    else if (NG == 4 && gr == 3) mg2l_group<P, GS, NG, NG == 4 ? 3 : 0>(row, g + qi, on, I, A);
-    else __syncthreads();
+    float2 L[Mg2lSplit<P>::most(NG)];
+    if (G == 0) mg2l_group_sums<P, GS, NG, 0>(row, g + qi, L, I);
+    else if (G == 1) mg2l_group_sums<P, GS, NG, 1>(row, g + qi, L, I);
+    else if (NG == 4 && G == 2) mg2l_group_sums<P, GS, NG, 2>(row, g + qi, L, I);
+    else if (NG == 4 && G == 3) mg2l_group_sums<P, GS, NG, 3>(row, g + qi, L, I);
+    __syncthreads();
+    if (G == 0) mg2l_group_store<P, NG, 0>(row, L, A);
+    else if (G == 1) mg2l_group_store<P, NG, 1>(row, L, A);
+    else if (NG == 4 && G == 2) mg2l_group_store<P, NG, 2>(row, L, A);
+    else if (NG == 4 && G == 3) mg2l_group_store<P, NG, 3>(row, L, A);
   }
 }
 
