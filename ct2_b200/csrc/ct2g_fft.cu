@@ -31,7 +31,8 @@ namespace {
 // output rows hold ld >= N/2+1 complex (the rest is written as zero).  VEC:
 // ld*sizeof(complex) is a multiple of 16 bytes.
 // (FP32 up to N = 256: four blocks per SM, whose loads and stores then overlap
-// the others' transforms; larger in-register DFTs and FP64 need the registers)
+// the others' transforms, at 64 registers, which spill 40 bytes a thread at N = 256; larger
+// in-register DFTs and FP64 need the registers)
 template <typename T, int N, bool VEC>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 && N <= 256 ? 4 : 3) fftz_r2c_kernel(const T *__restrict__ in,
                                                           typename Cplx<T>::type *__restrict__ out,

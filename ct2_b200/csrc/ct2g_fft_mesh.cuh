@@ -409,7 +409,8 @@ __device__ __forceinline__ void store_half_spectra(const float2 *s, float2 *rows
 }
 
 // occupancy: 4 blocks per SM up to order 4 (64 registers), 3 beyond on short lines
-// (2 where the lines fill the shared memory); at N = 512 the
+// (80 registers; from compact records order 6 spills 72-76 bytes there; 2 where the lines fill the
+// shared memory); at N = 512 the
 // 32-point in-register DFTs need more registers than that, so 2
 template <int P, int N, int SRC>
 __global__ void __launch_bounds__(256, N >= 512 ? 2 : P <= 4 ? 4 : N <= 128 ? 3 : 2) fftz_p2m_r2c_kernel(
@@ -817,7 +818,8 @@ struct PipeShape {
   static constexpr size_t ZS = (size_t)NL * LineLayout<N, true>::LS;  // a z line's packed lines
   static constexpr size_t YS = (size_t)N * kPipeW;                    // a y tile
   static constexpr size_t SMEM = sizeof(float2) * ((size_t)N + (ZS > YS ? ZS : YS));
-  // the z kernels' register budgets: 64 per thread up to order 4
+  // the z kernels' register budgets: 64 per thread up to order 4 (the y tiles' DFTs on top
+  // spill 8-228 bytes there)
   static constexpr int MINB = P <= 4 ? 4 : 2;
   static constexpr bool OK = N >= 64 && N <= 256;
 };

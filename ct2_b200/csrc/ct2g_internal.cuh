@@ -253,7 +253,8 @@ struct ct2g_ctx {
   unsigned long long *stmask = nullptr;  // [64][27] stencil bits per (in-block cell, block offset)
   float4 *src = nullptr;           // per sorted particle: offset from own cell centre
   uint2 *chunks = nullptr;         // near-field dense chunks (particle index, sinks)
-  uint32_t *sparse_list = nullptr; // particles of sparse cells, in order
+  uint32_t *sparse_list = nullptr; // particles of sparse cells (tiles of 2048 cells in any
+                                   // order, cell order within one)
   uint32_t *flags = nullptr;
   // work-list sizes stay on the device, so a step needs no host readback:
   // [0] dense chunks, [1] sparse sinks, [2] sparse chunks, [5] scan total

@@ -98,8 +98,8 @@ __device__ __forceinline__ int nth_set_bit(unsigned long long w, uint32_t r) {
 }
 
 // ---------------------------------------------------------------------------
-// Streamed near field.  A chunk is <= 32 sinks, one per lane: sinks of one
-// cell (dense), or the sparse cells' sinks of one 4x4x4 block (sparse).  Its
+// Streamed near field.  A chunk is sinks of one cell (dense: up to 64, one or two
+// per lane) or the sparse cells' sinks of one 4x4x4 block (sparse: up to 32, one per lane).  Its
 // candidate cells (occupancy & the union of its sinks' stencil masks, lane o <
 // 27 holding neighbouring block o's word) go in windows of 32, a cell per
 // lane; the sources of a window form one stream, staged in batches of 32 and
@@ -128,9 +128,14 @@ __device__ __forceinline__ int nth_set_bit(unsigned long long w, uint32_t r) {
 // it: FMA pipe 71%, all issue slots used; two sinks per lane halve that share.
 // Against one warp per chunk, cells' sources in batches of their own half
 // blocks (dense), a table of stencil entries per lane in shared memory (sparse)
-// and scalar arithmetic cell by cell (sphere kernel), a step of 2.5 M particles in halos
-// 48.6 -> 42.5 ms, 50 k in spheres 1.14 -> 0.88, 300 k with the sphere kernel and
-// potentials 11.96 -> 6.45, 128^3 in Plummer spheres 11.87 -> 11.55.
+// and scalar arithmetic cell by cell (sphere kernel), the near field of 2.5 M particles in halos
+// (mesh 256, 7.7e10 interactions) takes 38.5 -> 33.2 ms, of 50 k in spheres (mesh 64) 478 -> 178
+// us, of 12 boxes of 30 k 1054 -> 686, of 128^3 in Plummer spheres (256) 3.48 -> 3.34 ms;
+// forces and potentials of 300 k in halos with the sphere kernel 7.7 -> 5.0 to
+// 12.6 -> 7.9 ms a call, by the particles.
+// Register bounds: 64 (sparse, four blocks of eight warps per SM) and 80 (three, dense and
+// heavy) spill 4-24 and 8-16 bytes a thread, the sparse sphere kernel with potentials 152;
+// three blocks per SM instead (28 bytes) measured the same, 6.16 and 6.15 ms a call of the above.
 // ---------------------------------------------------------------------------
 struct NearArgs {
   const uint2 *dchunks;     // dense chunks (first particle, sinks), *ndense of them
@@ -166,9 +171,13 @@ struct NearArgs {
 // halos).  A block per chunk costs its eight warps the setup, so that it only
 // pays where a warp's chunk is long against the launch: a mesh of M has (M/4)^3
 // blocks, under one round of the GPU's warps up to 64, 7 at 128, 55 at 256.
-// Limits of 1024 / 3072 / 8192 / 16384 measured 0.88 / 0.95 / 1.04 / 1.04 ms a step
-// (50 k particles, mesh 64), 2.75 / 2.82 / 2.96 / 2.96 (262 k, 128, with the learned
-// correction), 11.9 / 11.75 / 11.58 / 11.52 (2.1 M, 256).
+// Near field in ms at limits of 1024 / 4096 / 8192 / 16384 / none: 50 k particles, mesh
+// 64, 0.180 / 0.287 / 0.351 / 0.358 / 0.354; 12 such boxes of 30 k (the boxes' blocks in all
+// do not matter: each box has its long chunks) 0.68 / 0.76 / 0.85 / 0.91 / 0.91; 2.1 M in
+// spheres, 256, 3.66 / 3.42 / 3.35 / 3.35 / 3.35; 4 M in spheres, 512, 6.07 / 4.74 / 4.56 / 4.56 / 4.57;
+// 4 M in halos, 512, 29.96 / 29.95 / 30.00 / 29.99 / 29.93.  Steps with the learned
+// correction (262 k, 128) 2.75 / 2.82 (3072) / 2.96 / 2.96.  From 256 on any limit of 8192 or
+// more measures the same; 8192 keeps one warp below some 80 us in sets that were not measured.
 uint32_t heavy_min(int M) { return M <= 128 ? 1024u : 8192u; }
 // SPLIT: the sparse sinks of the sphere kernel.  A coordinate in the frame of a
 // 4-cell block has lost up to three bits of the offset from its own cell's centre, so that
@@ -818,7 +827,7 @@ __device__ __forceinline__ void cells_chunk(const NearArgs &A, const uint2 cd, f
       }
     }
   }
-  if (act) {  // as near_chunk
+  if (act) {  // as write_sink
     const float gx = __fmul_rn(GM, nx), gy = __fmul_rn(GM, ny), gz = __fmul_rn(GM, nz);
     if (A.store) {
       A.ofx[i] = gx;
@@ -852,7 +861,8 @@ __global__ void __launch_bounds__(256, 4) near_cells_kernel(const NearArgs A) {
 }
 
 // Sparse sinks, one per lane: the warp takes 32 consecutive entries of the
-// sparse sink list (cell order, so the lanes are neighbours) and every lane
+// sparse sink list (cell order within a tile of 2048 cells, so that the lanes are
+// mostly neighbours; the tiles in any order) and every lane
 // walks the stencil of its own cell -- the 27 neighbouring 4x4x4 blocks,
 // occupancy & its own stencil mask, the ranges of the occupied cells -- and
 // sums its own sources, read through the read-only cache, two at a time with
@@ -953,7 +963,7 @@ __global__ void __launch_bounds__(256, 4) near_lane_kernel(
         }
       }
       // added to the far field already in the force buffers, or stored (the
-      // product rounded on its own, as in near_chunk)
+      // product rounded on its own, as in write_sink)
       const float gx = __fmul_rn(GM, nx), gy = __fmul_rn(GM, ny), gz = __fmul_rn(GM, nz);
       if (store) {
         ofx[i] = gx;

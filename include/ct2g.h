@@ -253,7 +253,9 @@ int ct2g_batch_destroy(ct2g_batch *b);
  * the Green's values straight from HBM inside the contraction instead of
  * staging each column in shared memory first (one more block per SM; the
  * same results); near_chunks_per_warp -- with overlap, > 0: a near-field warp
- * takes at most this many sink chunks before its block exits, so that the
+ * (or the warps that share a sparse chunk) takes at most this many sink
+ * chunks, a block of the dense chunks' launch, whose eight warps share each
+ * chunk, eight times as many, before the block exits, so that the
  * mesh solve's blocks (on the context stream, which has the higher priority)
  * get SMs in between; 0: the near-field grid is persistent; plane_pipe --
  * D > 0 (up to 16): the forward z pass (with P2M) and y pass run as one

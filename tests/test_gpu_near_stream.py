@@ -1,8 +1,7 @@
 """The streamed near field against the FP64 restatement of the method, at the
 sizes where it changes form: few chunks (shared by several warps), chunks
 whose neighbourhood is heavy (shared by a block), partial batches, both
-kernels, and the smallest meshes (a mesh of 8 takes the sparse chunks cell by
-cell)."""
+kernels, and the smallest meshes."""
 import numpy as np
 import pytest
 
